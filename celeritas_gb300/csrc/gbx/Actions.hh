@@ -104,7 +104,7 @@ GBX_FUNCTION void pre_step(ParamsData const& p, StateData const& s, size_type sl
     }
     else
     {
-        step = s.interaction_mfp[slot] / total_macro_xs;
+        step = div(s.interaction_mfp[slot], total_macro_xs);
         size_type const eloss = phys.group().eloss_process;
         if (eloss != invalid_id)
         {
@@ -188,7 +188,7 @@ GBX_FUNCTION real_type calc_eloss(ParamsData const& p,
         {
             real_type const mass = p.particles[pid].mass;
             real_type const electron_mass = p.particles[p.electron_id].mass;
-            real_type const gamma = 1 + energy / mass;
+            real_type const gamma = 1 + div(energy, mass);
             real_type const bsq = beta_sq(mass, energy);
             real_type const two_mebsgs = 2 * electron_mass * bsq * ipow<2>(gamma);
             real_type max_energy_transfer;
@@ -198,9 +198,9 @@ GBX_FUNCTION real_type calc_eloss(ParamsData const& p,
             }
             else
             {
-                real_type mass_ratio = electron_mass / mass;
+                real_type mass_ratio = div(electron_mass, mass);
                 max_energy_transfer
-                    = two_mebsgs / (1 + mass_ratio * (2 * gamma + mass_ratio));
+                    = div(two_mebsgs, 1 + mass_ratio * (2 * gamma + mass_ratio));
             }
             real_type const max_energy = min_of(
                 real_type(cutoff_energy(p, mid, p.electron_id)), max_energy_transfer);
@@ -285,12 +285,12 @@ GBX_FUNCTION void field_setup(ParamsData const& p,
     size_type const pid = s.particle_id[slot];
     real_type const mass = p.particles[pid].mass;
     real_type const energy = s.energy[slot];
-    double const momentum = std::sqrt(double(momentum_sq(mass, energy)));
+    double const momentum = gbx::sqrt(double(momentum_sq(mass, energy)));
     UniformFieldEquation rhs;
     rhs.field = {p.field[0], p.field[1], p.field[2]};
     rhs.map = p.has_rzmap ? p.rzmap : nullptr;
-    rhs.coeffi = (p.particles[pid].charge * detail::e_electron)
-                 / (1 * (detail::mev_value / constants::c_light));
+    rhs.coeffi = div(p.particles[pid].charge * detail::e_electron,
+                     1 * (detail::mev_value / constants::c_light));
     fp->set_rhs(rhs);
     fp->init(geo, momentum, s.step_length[slot], start_safety);
 }
@@ -381,11 +381,11 @@ GBX_FUNCTION void along_epilogue(ParamsData const& p,
     {
         real_type const mass = p.particles[pid].mass;
         real_type const speed
-            = std::sqrt(beta_sq(mass, s.energy[slot])) * real_type(constants::c_light);
+            = gbx::sqrt(beta_sq(mass, s.energy[slot])) * real_type(constants::c_light);
         if (speed > 0)
         {
             // Time accumulates in FP64; the increment is a physics quantity
-            s.time[slot] += double(real_type(s.step_length[slot]) / speed);
+            s.time[slot] += double(div(real_type(s.step_length[slot]), speed));
         }
     }
 

@@ -48,18 +48,18 @@ GBX_FORCEINLINE double fastpow(double a, double b)
 GBX_FUNCTION Real3 rzmap_field(RZMapData const& m, Real3 const& pos)
 {
     Real3 value{0, 0, 0};
-    double const r = std::sqrt(ipow<2>(pos.x) + ipow<2>(pos.y));
+    double const r = gbx::sqrt(ipow<2>(pos.x) + ipow<2>(pos.y));
     if (!(pos.z >= m.z.front && pos.z <= m.z.back && r >= m.r.front && r <= m.r.back))
         return value;
     // find_interp on a uniform grid (UniformGrid::find, operator[]); a value
     // on the last node takes the last interval
     auto locate = [](FieldMapGrid const& g, double v, size_type* index) {
-        size_type i = static_cast<size_type>((v - g.front) / g.delta);
+        size_type i = static_cast<size_type>(div(v - g.front, g.delta));
         i = min_of(i, g.size - 2);
         double const lower = g.front + g.delta * i;
         double const upper = g.front + g.delta * (i + 1);
         *index = i;
-        return (v - lower) / (upper - lower);
+        return div(v - lower, upper - lower);
     };
     size_type ir, iz;
     double const fr = locate(m.r, r, &ir);
@@ -70,7 +70,7 @@ GBX_FUNCTION Real3 rzmap_field(RZMapData const& m, Real3 const& pos)
     value.z = low + (high - low) * fz;
     low = m.values[iz * nr + ir].value_r;
     high = m.values[iz * nr + ir + 1].value_r;
-    double const tmp = (r != 0) ? (low + (high - low) * fr) / r : low;
+    double const tmp = (r != 0) ? div(low + (high - low) * fr, r) : low;
     value.x = tmp * pos.x;
     value.y = tmp * pos.y;
     return value;
@@ -81,12 +81,12 @@ GBX_FUNCTION Real3 rzmap_field(RZMapData const& m, Real3 const& pos)
 GBX_NOINLINE Vec3<float> rzmap_field_f(RZMapData const& m, Vec3<float> const& pos)
 {
     Vec3<float> value{0, 0, 0};
-    float const r = std::sqrt(pos.x * pos.x + pos.y * pos.y);
+    float const r = gbx::sqrt(pos.x * pos.x + pos.y * pos.y);
     if (!(pos.z >= float(m.z.front) && pos.z <= float(m.z.back) && r >= float(m.r.front)
           && r <= float(m.r.back)))
         return value;
     auto locate = [](FieldMapGrid const& g, float v, size_type* index) {
-        float const u = (v - float(g.front)) / float(g.delta);
+        float const u = div(v - float(g.front), float(g.delta));
         size_type const i = min_of(static_cast<size_type>(u), g.size - 2);
         *index = i;
         return u - float(i);
@@ -101,7 +101,7 @@ GBX_NOINLINE Vec3<float> rzmap_field_f(RZMapData const& m, Vec3<float> const& po
     value.z = low + (high - low) * fz;
     low = v[iz * nr + ir].value_r;
     high = v[iz * nr + ir + 1].value_r;
-    float const tmp = (r != 0) ? (low + (high - low) * fr) / r : low;
+    float const tmp = (r != 0) ? div(low + (high - low) * fr, r) : low;
     value.x = tmp * pos.x;
     value.y = tmp * pos.y;
     return value;
@@ -118,7 +118,7 @@ struct UniformFieldEquation
 
     GBX_FORCEINLINE OdeState operator()(OdeState const& y) const
     {
-        double momentum_inv = 1.0 / std::sqrt(dot_product(y.mom, y.mom));
+        double momentum_inv = div(1.0, gbx::sqrt(dot_product(y.mom, y.mom)));
         OdeState result;
         result.pos = {momentum_inv * y.mom.x,
                       momentum_inv * y.mom.y,
@@ -151,7 +151,7 @@ struct FixedFieldEquation
 
     GBX_FORCEINLINE OdeState operator()(OdeState const& y) const
     {
-        double momentum_inv = 1.0 / std::sqrt(dot_product(y.mom, y.mom));
+        double momentum_inv = div(1.0, gbx::sqrt(dot_product(y.mom, y.mom)));
         OdeState result;
         result.pos = {momentum_inv * y.mom.x,
                       momentum_inv * y.mom.y,
@@ -298,7 +298,7 @@ GBX_FUNCTION FieldStepperResult dormand_prince_step_mixed(UniformFieldEquation c
         F3 const field
             = rhs.map ? rzmap_field_f(*rhs.map, F3{p0.x + dp.x, p0.y + dp.y, p0.z + dp.z})
                       : uniform;
-        F const inv = F(1) / std::sqrt(m.x * m.x + m.y * m.y + m.z * m.z);
+        F const inv = div(F(1), gbx::sqrt(m.x * m.x + m.y * m.y + m.z * m.z));
         *kpos = {m.x * inv, m.y * inv, m.z * inv};
         F const scale = coeffi * inv;
         *kmom = {scale * (m.y * field.z - m.z * field.y),
@@ -393,9 +393,9 @@ GBX_FUNCTION FieldStepperResult dormand_prince_step_mixed(UniformFieldEquation c
     F3 const cr{end_inc.y * mid_inc.z - end_inc.z * mid_inc.y,
                 end_inc.z * mid_inc.x - end_inc.x * mid_inc.z,
                 end_inc.x * mid_inc.y - end_inc.y * mid_inc.x};
-    result.dchord = std::sqrt((cr.x * cr.x + cr.y * cr.y + cr.z * cr.z)
-                              / (end_inc.x * end_inc.x + end_inc.y * end_inc.y
-                                 + end_inc.z * end_inc.z));
+    result.dchord = gbx::sqrt(div(cr.x * cr.x + cr.y * cr.y + cr.z * cr.z,
+                                  end_inc.x * end_inc.x + end_inc.y * end_inc.y
+                                      + end_inc.z * end_inc.z));
     return result;
 }
 
@@ -489,8 +489,8 @@ class FieldDriver
     {
         double errpos2 = dot_product(err_state.pos, err_state.pos);
         double errvel2 = dot_product(err_state.mom, err_state.mom);
-        errpos2 /= ipow<2>(step);
-        errvel2 /= dot_product(mom, mom);
+        errpos2 = div(errpos2, ipow<2>(step));
+        errvel2 = div(errvel2, dot_product(mom, mom));
         return max_of(errpos2, errvel2);
     }
 
@@ -501,8 +501,8 @@ class FieldDriver
     {
         if constexpr (sizeof(real_type) == sizeof(double))
         {
-            return rel_err_sq(result.err_state, step, mom)
-                   / ipow<2>(opt_.epsilon_rel_max);
+            return div(rel_err_sq(result.err_state, step, mom),
+                       ipow<2>(opt_.epsilon_rel_max));
         }
         else
         {
@@ -515,8 +515,8 @@ class FieldDriver
                            double(result.err_mom.y),
                            double(result.err_mom.z)};
             double const errpos2 = dot_product(ep, ep);
-            double const errvel2 = dot_product(em, em) / dot_product(mom, mom);
-            return max_of(errpos2, errvel2) / ipow<2>(opt_.epsilon_rel_max);
+            double const errvel2 = div(dot_product(em, em), dot_product(mom, mom));
+            return div(max_of(errpos2, errvel2), ipow<2>(opt_.epsilon_rel_max));
         }
     }
 
@@ -537,7 +537,7 @@ class FieldDriver
         Real3 beg_mid{mid_pos.x - beg_pos.x, mid_pos.y - beg_pos.y, mid_pos.z - beg_pos.z};
         Real3 beg_end{end_pos.x - beg_pos.x, end_pos.y - beg_pos.y, end_pos.z - beg_pos.z};
         Real3 cross = cross_product(beg_end, beg_mid);
-        return std::sqrt(dot_product(cross, cross) / dot_product(beg_end, beg_end));
+        return gbx::sqrt(div(dot_product(cross, cross), dot_product(beg_end, beg_end)));
     }
 
     GBX_FORCEINLINE double new_step_scale(double err_sq) const
@@ -568,7 +568,7 @@ class FieldDriver
             double dchord = this->chord_distance(result, state);
             if (dchord > opt_.delta_chord + FieldOptions::dchord_tol)
             {
-                double scale_step = max_of(std::sqrt(opt_.delta_chord / dchord),
+                double scale_step = max_of(gbx::sqrt(div(opt_.delta_chord, dchord)),
                                            FieldOptions::min_chord_shrink);
                 step *= scale_step;
             }
@@ -734,14 +734,14 @@ class FieldPropagation
         double const clen = norm(cdir);
         if constexpr (sizeof(real_type) == sizeof(double))
         {
-            cdir.x /= clen;
-            cdir.y /= clen;
-            cdir.z /= clen;
+            cdir.x = div(cdir.x, clen);
+            cdir.y = div(cdir.y, clen);
+            cdir.z = div(cdir.z, clen);
         }
         else
         {
             // One FP64 division instead of three
-            double const inv_clen = 1 / clen;
+            double const inv_clen = div(1, clen);
             cdir.x *= inv_clen;
             cdir.y *= inv_clen;
             cdir.z *= inv_clen;
@@ -781,7 +781,7 @@ class FieldPropagation
             return;
         }
         // Scaled length of the chord up to the crossing (only with one)
-        double const update_length = substep.step * linear_step.distance / clen;
+        double const update_length = div(substep.step * linear_step.distance, clen);
         auto is_intercept_close = [&]() {
             double delta_sq = 0;
             for (int i = 0; i < 3; ++i)

@@ -235,7 +235,7 @@ class GeoTrackView
             double const n_dir = dir[sr.type];
             if (n_dir != 0)
             {
-                double const d = (sr.value - pos[sr.type]) / n_dir;
+                double const d = div(sr.value - pos[sr.type], n_dir);
                 if (d > 0)
                     dist[0] = d;
             }
@@ -267,7 +267,7 @@ class GeoTrackView
         if (a < ipow<2>(sqrt_quadratic))
             return;
         double const half_b = dir.x * pos.x + dir.y * pos.y;
-        double const a_inv = 1 / a;
+        double const a_inv = div(1, a);
         double const hba = half_b * a_inv;
         if (on_surface)
         {
@@ -280,7 +280,7 @@ class GeoTrackView
         double const b2_4 = ipow<2>(hba);
         if (b2_4 > c)
         {
-            double const t2 = std::sqrt(b2_4 - c);
+            double const t2 = gbx::sqrt(b2_4 - c);
             double const r0 = -hba - t2;
             double const r1 = -hba + t2;
             if (r1 > 0)
@@ -344,7 +344,7 @@ class GeoTrackView
             double const q = rsq - sr.value;
             if (q == 0)
                 return 0;
-            return std::fabs(std::sqrt(rsq) - sr.radius_d);
+            return std::fabs(gbx::sqrt(rsq) - sr.radius_d);
         }
         Real3 n = make_unit_vector(Real3{pos.x, pos.y, 0});
         if (std::isnan(n.x))
@@ -721,7 +721,7 @@ GBX_FUNCTION void GeoTrackView::background_crossing(Real3 const& pos,
     {
         float const xf = static_cast<float>(pos.x);
         float const yf = static_cast<float>(pos.y);
-        float const rf = std::sqrt(xf * xf + yf * yf);
+        float const rf = gbx::sqrt(xf * xf + yf * yf);
         auto radial_margin = [](float radius, float limit) {
             return 1e-5f * (radius + limit) + 1e-6f;
         };
@@ -810,7 +810,7 @@ GBX_FUNCTION void GeoTrackView::background_crossing(Real3 const& pos,
                     continue;
                 if (gap * (1 - 0x1p-40) > crossing_limit(*hit))
                     break;
-                double const d = gap / n;
+                double const d = div(gap, n);
                 if (d > 0)
                     this->consider_crossing(surf, d, pos, dir, bump, max_step, hit);
             }
@@ -826,7 +826,7 @@ GBX_FUNCTION void GeoTrackView::background_crossing(Real3 const& pos,
                     continue;
                 if (-gap * (1 - 0x1p-40) > crossing_limit(*hit))
                     break;
-                double const d = gap / n;
+                double const d = div(gap, n);
                 if (d > 0)
                     this->consider_crossing(surf, d, pos, dir, bump, max_step, hit);
             }
@@ -948,7 +948,7 @@ GBX_FUNCTION double GeoTrackView::find_safety() const
     // is unchanged, and far cylinders cost a few FP32 operations.
     float const xf = static_cast<float>(pos.x);
     float const yf = static_cast<float>(pos.y);
-    float const rf = std::sqrt(xf * xf + yf * yf);
+    float const rf = gbx::sqrt(xf * xf + yf * yf);
     auto visit = [&](size_type surf) {
         SurfaceRecord const& sr = p_.surfaces[surf];
         if (sr.type == surf_czc)

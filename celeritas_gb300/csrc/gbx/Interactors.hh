@@ -100,7 +100,7 @@ GBX_FORCEINLINE real_type sample_tsai_urban(real_type energy,
                                             real_type mass,
                                             G& rng)
 {
-    real_type const umax = 2 * (1 + energy / mass);
+    real_type const umax = 2 * (1 + div(energy, mass));
     real_type u;
     do
     {
@@ -111,7 +111,7 @@ GBX_FORCEINLINE real_type sample_tsai_urban(real_type energy,
                    ? real_type(1.6)
                    : real_type(1.6 / 3));
     } while (u > umax);
-    return 1 - 2 * ipow<2>(u / umax);
+    return 1 - 2 * ipow<2>(div(u, umax));
 }
 
 //---------------------------------------------------------------------------//
@@ -129,9 +129,9 @@ GBX_FUNCTION Interaction interact_klein_nishina(ParamsData const& p,
         return Interaction::from_failure();
 
     real_type const inv_electron_mass
-        = real_type(1 / p.particles[p.electron_id].mass);
+        = real_type(div(1, p.particles[p.electron_id].mass));
     real_type const k = inc_energy * inv_electron_mass;
-    real_type const epsilon_0 = 1 / (1 + 2 * k);
+    real_type const epsilon_0 = div(1, 1 + 2 * k);
     real_type const p_f1 = bernoulli_p(-libm::log(epsilon_0),
                                        real_type(0.5) * (1 - ipow<2>(epsilon_0)));
     ReciprocalDistribution<real_type> sample_f1(1, epsilon_0);
@@ -151,11 +151,11 @@ GBX_FUNCTION Interaction interact_klein_nishina(ParamsData const& p,
         else
         {
             epsilon_sq = sample_f2_sq(rng);
-            epsilon = std::sqrt(epsilon_sq);
+            epsilon = gbx::sqrt(epsilon_sq);
         }
-        one_minus_costheta = (1 - epsilon) / (epsilon * k);
+        one_minus_costheta = div(1 - epsilon, epsilon * k);
         real_type sintheta_sq = one_minus_costheta * (2 - one_minus_costheta);
-        reject_prob = epsilon * sintheta_sq / (1 + epsilon_sq);
+        reject_prob = div(epsilon * sintheta_sq, 1 + epsilon_sq);
     } while (sample_bernoulli<real_type>(reject_prob, rng));
 
     Interaction result;
@@ -195,9 +195,9 @@ GBX_FUNCTION Interaction interact_livermore_pe(ParamsData const& p,
 
     LivermoreElement const& el = p.livermore_elements[element];
     LivermoreShell const* shells = p.livermore_shells + el.shells;
-    real_type const inv_energy = 1 / inc_energy;
+    real_type const inv_energy = div(1, inc_energy);
     real_type const inv_electron_mass
-        = real_type(1 / p.particles[p.electron_id].mass);
+        = real_type(div(1, p.particles[p.electron_id].mass));
 
     // Sample the subshell
     size_type shell_id = 0;
@@ -250,19 +250,18 @@ GBX_FUNCTION Interaction interact_livermore_pe(ParamsData const& p,
         real_type energy_per_mecsq = max_of(real_type(1.e-6), inc_energy)
                                      * inv_electron_mass;
         real_type gamma = energy_per_mecsq + 1;
-        real_type beta = std::sqrt(energy_per_mecsq * (gamma + 1)) / gamma;
-        real_type a = (1 - beta) / beta;
+        real_type beta = div(gbx::sqrt(energy_per_mecsq * (gamma + 1)), gamma);
+        real_type a = div(1 - beta, beta);
         constexpr real_type half = 0.5;
         real_type b = half * beta * gamma * energy_per_mecsq * (gamma - 2);
-        real_type g_max = 2 * (1 / a + b);
+        real_type g_max = 2 * (div(1, a) + b);
         real_type g;
         real_type nu;
         do
         {
             real_type u = generate_canonical<real_type>(rng);
-            nu = 2 * a * (2 * u + (a + 2) * std::sqrt(u))
-                 / (ipow<2>(a + 2) - 4 * u);
-            g = (2 - nu) * (1 / (a + nu) + b);
+            nu = div(2 * a * (2 * u + (a + 2) * gbx::sqrt(u)), ipow<2>(a + 2) - 4 * u);
+            g = (2 - nu) * (div(1, a + nu) + b);
         } while (g < g_max * generate_canonical<real_type>(rng));
         edir = sample_exiting_direction<real_type>(1 - nu, inc_dir, rng);
     }
@@ -306,7 +305,7 @@ GBX_FUNCTION Interaction interact_bethe_heitler(ParamsData const& p,
         return Interaction::from_failure();
 
     real_type const electron_mass = p.particles[p.electron_id].mass;
-    real_type const epsilon0 = electron_mass / inc_energy;
+    real_type const epsilon0 = div(electron_mass, inc_energy);
     real_type const cbrt_z = element.cbrt_z;
     constexpr real_type half = 0.5;
     real_type epsilon;
@@ -316,24 +315,24 @@ GBX_FUNCTION Interaction interact_bethe_heitler(ParamsData const& p,
     }
     else
     {
-        real_type const delta_min = 4 * 136 / cbrt_z * epsilon0;
+        real_type const delta_min = div(4 * 136, cbrt_z) * epsilon0;
         real_type f_z = real_type(8) / real_type(3) * real_type(element.log_z);
         if (inc_energy > real_type(50))
         {
             f_z += 8 * real_type(element.coulomb_correction);
         }
         real_type const delta_max
-            = libm::exp((real_type(42.038) - f_z) / real_type(8.29))
+            = libm::exp(div(real_type(42.038) - f_z, real_type(8.29)))
               - real_type(0.958);
         real_type const epsilon1
-            = half - half * std::sqrt(1 - delta_min / delta_max);
+            = half - half * gbx::sqrt(1 - div(delta_min, delta_max));
         real_type const epsilon_min = max_of(epsilon0, epsilon1);
         real_type const f10 = bh_screening_f1(delta_min) - f_z;
         real_type const f20 = bh_screening_f2(delta_min) - f_z;
         real_type const p_f1g1
             = bernoulli_p(ipow<2>(half - epsilon_min) * f10, real_type(1.5) * f20);
         auto impact_parameter = [&](real_type eps) {
-            return 136 / cbrt_z * epsilon0 / (eps * (1 - eps));
+            return div(div(136, cbrt_z) * epsilon0, eps * (1 - eps));
         };
         real_type g;
         do
@@ -344,14 +343,14 @@ GBX_FUNCTION Interaction interact_bethe_heitler(ParamsData const& p,
                           - (half - epsilon_min)
                                 * libm::cbrt(generate_canonical<real_type>(rng));
                 real_type delta = impact_parameter(epsilon);
-                g = (bh_screening_f1(delta) - f_z) / f10;
+                g = div(bh_screening_f1(delta) - f_z, f10);
             }
             else
             {
                 epsilon = epsilon_min
                           + (half - epsilon_min) * generate_canonical<real_type>(rng);
                 real_type delta = impact_parameter(epsilon);
-                g = (bh_screening_f2(delta) - f_z) / f20;
+                g = div(bh_screening_f2(delta) - f_z, f20);
             }
         } while (g < generate_canonical<real_type>(rng));
     }
@@ -405,7 +404,7 @@ struct SBXsCalc
         size_type iy = find_nonuniform(ygrid, t.ny, y);
         real_type const lower = ygrid[iy];
         real_type const upper = ygrid[iy + 1];
-        real_type const yf = (y - lower) / (upper - lower);
+        real_type const yf = div(y - lower, upper - lower);
         real_type const xf = x_fraction;
         return (1 - xf) * ((1 - yf) * at(x_index, iy) + (yf)*at(x_index, iy + 1))
                + (xf) * ((1 - yf) * at(x_index + 1, iy) + (yf)*at(x_index + 1, iy + 1));
@@ -429,7 +428,7 @@ GBX_FUNCTION Interaction interact_seltzer_berger(ParamsData const& p,
         return Interaction::from_failure();
 
     real_type const inc_momentum
-        = std::sqrt(momentum_sq(inc_mass, inc_energy));
+        = gbx::sqrt(momentum_sq(inc_mass, inc_energy));
     // Density (dielectric suppression) correction
     constexpr real_type migdal = 4 * constants::pi * constants::r_electron
                                  * ipow<2>(constants::lambdabar_electron);
@@ -442,8 +441,8 @@ GBX_FUNCTION Interaction interact_seltzer_berger(ParamsData const& p,
     real_type const* xgrid = p.reals + t.x;
     real_type const loge = libm::log(inc_energy);
     size_type ix = find_nonuniform(xgrid, t.nx, loge);
-    real_type const xf = (loge - real_type(xgrid[ix]))
-                         / (real_type(xgrid[ix + 1]) - real_type(xgrid[ix]));
+    real_type const xf = div(loge - real_type(xgrid[ix]),
+                             real_type(xgrid[ix + 1]) - real_type(xgrid[ix]));
     SBXsCalc calc_xs{p, t, ix, xf};
     real_type max_xs;
     {
@@ -453,7 +452,7 @@ GBX_FUNCTION Interaction interact_seltzer_berger(ParamsData const& p,
         };
         max_xs = (1 - xf) * get_value(ix) + xf * get_value(ix + 1);
     }
-    real_type const inv_inc_energy = 1 / inc_energy;
+    real_type const inv_inc_energy = div(1, inc_energy);
     ReciprocalDistribution<real_type> sample_exit_esq(
         ipow<2>(gamma_cutoff) + dens_corr, ipow<2>(inc_energy) + dens_corr);
 
@@ -463,7 +462,7 @@ GBX_FUNCTION Interaction interact_seltzer_berger(ParamsData const& p,
                               * real_type(p.elements[element_id].z);
     auto calc_invbeta = [&](real_type gamma_energy) {
         real_type energy = inc_energy - gamma_energy;
-        return (energy + inc_mass) / std::sqrt(energy * (energy + 2 * inc_mass));
+        return div(energy + inc_mass, gbx::sqrt(energy * (energy + 2 * inc_mass)));
     };
     real_type const cutoff_invbeta = is_electron ? 0 : calc_invbeta(gamma_cutoff);
 
@@ -472,7 +471,7 @@ GBX_FUNCTION Interaction interact_seltzer_berger(ParamsData const& p,
     do
     {
         real_type esq = sample_exit_esq(rng) - dens_corr;
-        gamma_energy = std::sqrt(esq);
+        gamma_energy = gbx::sqrt(esq);
         xs = calc_xs(gamma_energy * inv_inc_energy);
         if (is_electron)
         {
@@ -549,9 +548,9 @@ GBX_FUNCTION LPMFunctions calc_lpm(MaterialRecord const& mat,
 {
     constexpr real_type sqrt_two = 1.41421356237309504880;
     real_type const lpm_energy = real_type(mat.rad_length) * real_type(lpm_constant());
-    real_type const s_prime = std::sqrt(
-        lpm_energy / (8 * epsilon * gamma_energy * std::fabs(epsilon - 1)));
-    real_type const s1 = ipow<2>(real_type(el.cbrt_z) / real_type(184.15));
+    real_type const s_prime = gbx::sqrt(
+        div(lpm_energy, 8 * epsilon * gamma_energy * std::fabs(epsilon - 1)));
+    real_type const s1 = ipow<2>(div(real_type(el.cbrt_z), real_type(184.15)));
     real_type xi = 2;
     if (s_prime > 1)
     {
@@ -560,16 +559,16 @@ GBX_FUNCTION LPMFunctions calc_lpm(MaterialRecord const& mat,
     else if (s_prime > sqrt_two * s1)
     {
         real_type const log_s1 = libm::log(sqrt_two * s1);
-        real_type const h = libm::log(s_prime) / log_s1;
-        xi = 1 + h - real_type(0.08) * (1 - h) * h * (2 - h) / log_s1;
+        real_type const h = div(libm::log(s_prime), log_s1);
+        xi = 1 + h - div(real_type(0.08) * (1 - h) * h * (2 - h), log_s1);
     }
-    real_type s = s_prime / std::sqrt(xi);
+    real_type s = div(s_prime, gbx::sqrt(xi));
     // Dielectric suppression is always on for relativistic bremsstrahlung
     {
         real_type const k_p_sq = real_type(mat.electron_density)
                                  * real_type(migdal_constant())
                                  * ipow<2>(epsilon * gamma_energy);
-        s *= (1 + k_p_sq / ipow<2>(gamma_energy));
+        s *= (1 + div(k_p_sq, ipow<2>(gamma_energy)));
         xi = 2;
         if (s > 1)
         {
@@ -577,7 +576,7 @@ GBX_FUNCTION LPMFunctions calc_lpm(MaterialRecord const& mat,
         }
         else if (s > s1)
         {
-            xi = 1 + libm::log(s) / libm::log(s1);
+            xi = 1 + div(libm::log(s), libm::log(s1));
         }
     }
     real_type phi;
@@ -591,17 +590,17 @@ GBX_FUNCTION LPMFunctions calc_lpm(MaterialRecord const& mat,
         real_type const ca[3] = {real_type(0.623), real_type(0.796), real_type(0.658)};
         real_type a = poly_eval<2>(ca, s);
         real_type const cb[3]
-            = {real_type(-6), real_type(-6 * (3 - constants::pi)), 1 / a};
+            = {real_type(-6), real_type(-6 * (3 - constants::pi)), div(1, a)};
         real_type b = poly_eval<2>(cb, s);
         phi = 1 - libm::exp(s * b);
     }
     else
     {
-        phi = 1 - real_type(0.01190476) / ipow<4>(s);
+        phi = 1 - div(real_type(0.01190476), ipow<4>(s));
     }
     if (xi * phi > 1 || s > real_type(0.57))
     {
-        xi = 1 / phi;
+        xi = div(1, phi);
     }
     real_type g;
     if (s < real_type(0.01))
@@ -617,7 +616,7 @@ GBX_FUNCTION LPMFunctions calc_lpm(MaterialRecord const& mat,
                                  real_type(-0.05),
                                  real_type(7.5)};
         real_type a = poly_eval<4>(ca, s);
-        real_type const cb[2] = {real_type(-4), -8 / a};
+        real_type const cb[2] = {real_type(-4), div(-8, a)};
         real_type b = poly_eval<1>(cb, s);
         real_type psi = 1 - libm::exp(s * b);
         g = 3 * psi - 2 * phi;
@@ -633,7 +632,7 @@ GBX_FUNCTION LPMFunctions calc_lpm(MaterialRecord const& mat,
     }
     else
     {
-        g = 1 - real_type(0.0230655) / ipow<4>(s);
+        g = 1 - div(real_type(0.0230655), ipow<4>(s));
     }
     return {xi, g, phi};
 }
@@ -656,18 +655,18 @@ GBX_FUNCTION Interaction interact_relativistic_brems(ParamsData const& p,
     using R = real_type;
     RelBremElementRecord const& ed = p.rb_elements[element_id];
     ElementRecord const& el = p.elements[element_id];
-    real_type const inc_momentum = std::sqrt(momentum_sq(inc_mass, inc_energy));
+    real_type const inc_momentum = gbx::sqrt(momentum_sq(inc_mass, inc_energy));
     real_type const total_energy = inc_energy + inc_mass;
     real_type const density_factor
         = R(mat.electron_density) * R(detail::migdal_constant());
     real_type const density_corr = density_factor * ipow<2>(total_energy);
     real_type const lpm_energy = R(mat.rad_length) * R(detail::lpm_constant());
-    real_type const lpm_threshold = lpm_energy * std::sqrt(density_factor);
+    real_type const lpm_threshold = lpm_energy * gbx::sqrt(density_factor);
     bool const enable_lpm = p.enable_lpm && (total_energy > lpm_threshold);
 
     auto dxsec_per_atom = [&](real_type gamma_energy) -> real_type {
         real_type dxsec{0};
-        real_type y = gamma_energy / total_energy;
+        real_type y = div(gamma_energy, total_energy);
         real_type onemy = 1 - y;
         real_type term0 = onemy + R(0.75) * ipow<2>(y);
         if (el.z < 5)
@@ -676,8 +675,8 @@ GBX_FUNCTION Interaction interact_relativistic_brems(ParamsData const& p,
         }
         else
         {
-            real_type invz = 1 / static_cast<real_type>(el.z);
-            real_type term1 = y / (total_energy - gamma_energy);
+            real_type invz = div(1, static_cast<real_type>(el.z));
+            real_type term1 = div(y, total_energy - gamma_energy);
             real_type gam = term1 * R(ed.gamma_factor);
             real_type eps = term1 * R(ed.epsilon_factor);
             real_type gam2 = ipow<2>(gam);
@@ -685,22 +684,22 @@ GBX_FUNCTION Interaction interact_relativistic_brems(ParamsData const& p,
             real_type phi1 = R(16.863) - 2 * libm::log(1 + R(0.311877) * gam2)
                              + R(2.4) * libm::exp(R(-0.9) * gam)
                              + R(1.6) * libm::exp(R(-1.5) * gam);
-            real_type phi2 = 2 / (3 + R(19.5) * gam + 18 * gam2);
+            real_type phi2 = div(2, 3 + R(19.5) * gam + 18 * gam2);
             real_type psi1 = R(24.34) - 2 * libm::log(1 + R(13.111641) * eps2)
                              + R(2.8) * libm::exp(R(-8) * eps)
                              + R(1.2) * libm::exp(R(-29.2) * eps);
-            real_type psi2 = 2 / (3 + 120 * eps + 1200 * eps2);
+            real_type psi2 = div(2, 3 + 120 * eps + 1200 * eps2);
             dxsec = term0
                         * ((R(0.25) * phi1 - R(ed.fz))
-                           + (R(0.25) * psi1 - 2 * R(el.log_z) / 3) * invz)
+                           + (R(0.25) * psi1 - div(2 * R(el.log_z), 3)) * invz)
                     + R(0.125) * onemy * (phi2 + psi2 * invz);
         }
         return max_of(dxsec, R(0));
     };
     auto dxsec_per_atom_lpm = [&](real_type gamma_energy) -> real_type {
-        real_type epsilon = total_energy / gamma_energy;
+        real_type epsilon = div(total_energy, gamma_energy);
         detail::LPMFunctions lpm = detail::calc_lpm(mat, el, gamma_energy, epsilon);
-        real_type y = gamma_energy / total_energy;
+        real_type y = div(gamma_energy, total_energy);
         real_type onemy = 1 - y;
         real_type y2 = R(0.25) * ipow<2>(y);
         real_type term = lpm.xi * (y2 * lpm.g + (onemy + 2 * y2) * lpm.phi);
@@ -718,7 +717,7 @@ GBX_FUNCTION Interaction interact_relativistic_brems(ParamsData const& p,
     real_type dsigma{0};
     do
     {
-        gamma_energy = std::sqrt(sample_exit_esq(rng) - density_corr);
+        gamma_energy = gbx::sqrt(sample_exit_esq(rng) - density_corr);
         dsigma = enable_lpm ? dxsec_per_atom_lpm(gamma_energy)
                             : dxsec_per_atom(gamma_energy);
     } while (reject_sample<real_type>(dsigma, max_value, rng));
@@ -755,41 +754,41 @@ GBX_FUNCTION Interaction interact_moller_bhabha(ParamsData const& p,
 
     real_type const electron_mass = p.particles[p.electron_id].mass;
     real_type const inc_momentum
-        = std::sqrt(momentum_sq(electron_mass, inc_energy));
-    real_type const min_energy_fraction = electron_cutoff / inc_energy;
-    real_type const gamma = 1 + inc_energy / electron_mass;
+        = gbx::sqrt(momentum_sq(electron_mass, inc_energy));
+    real_type const min_energy_fraction = div(electron_cutoff, inc_energy);
+    real_type const gamma = 1 + div(inc_energy, electron_mass);
     real_type epsilon;
     if (is_electron)
     {
         auto calc_g_fraction = [gamma](real_type eps) {
-            real_type const two_gamma_term = (2 * gamma - 1) / ipow<2>(gamma);
+            real_type const two_gamma_term = div(2 * gamma - 1, ipow<2>(gamma));
             real_type const complement_frac = 1 - eps;
             return 1 - two_gamma_term * eps
                    + ipow<2>(eps)
                          * (1 - two_gamma_term
-                            + (1 - two_gamma_term * complement_frac)
-                                  / ipow<2>(complement_frac));
+                            + div(1 - two_gamma_term * complement_frac,
+                                  ipow<2>(complement_frac)));
         };
         constexpr real_type max_energy_fraction = 0.5;
         real_type const g_denominator = calc_g_fraction(max_energy_fraction);
         UniformRealDistribution<real_type> sample_inverse_epsilon(
-            1 / max_energy_fraction, 1 / min_energy_fraction);
+            div(1, max_energy_fraction), div(1, min_energy_fraction));
         do
         {
-            epsilon = 1 / sample_inverse_epsilon(rng);
+            epsilon = div(1, sample_inverse_epsilon(rng));
         } while (reject_sample<real_type>(calc_g_fraction(epsilon), g_denominator, rng));
     }
     else
     {
         auto calc_g_fraction = [gamma](real_type eps_min, real_type eps_max) {
-            real_type const y = 1 / (1 + gamma);
+            real_type const y = div(1, 1 + gamma);
             real_type const y_sq = ipow<2>(y);
             real_type const one_minus_2y = 1 - 2 * y;
             real_type const b1 = 2 - y_sq;
             real_type const b2 = one_minus_2y * (3 + y_sq);
             real_type const b4 = ipow<3>(one_minus_2y);
             real_type const b3 = ipow<2>(one_minus_2y) + b4;
-            real_type const beta_sq = 1 - (1 / ipow<2>(gamma));
+            real_type const beta_sq = 1 - div(1, ipow<2>(gamma));
             return 1
                    + (ipow<4>(eps_max) * b4 - ipow<3>(eps_min) * b3
                       + ipow<2>(eps_max) * b2 - eps_min * b1)
@@ -799,10 +798,10 @@ GBX_FUNCTION Interaction interact_moller_bhabha(ParamsData const& p,
         real_type const g_denominator
             = calc_g_fraction(min_energy_fraction, max_energy_fraction);
         UniformRealDistribution<real_type> sample_inverse_epsilon(
-            1 / max_energy_fraction, 1 / min_energy_fraction);
+            div(1, max_energy_fraction), div(1, min_energy_fraction));
         do
         {
-            epsilon = 1 / sample_inverse_epsilon(rng);
+            epsilon = div(1, sample_inverse_epsilon(rng));
         } while (reject_sample<real_type>(
             calc_g_fraction(epsilon, epsilon), g_denominator, rng));
     }
@@ -810,10 +809,10 @@ GBX_FUNCTION Interaction interact_moller_bhabha(ParamsData const& p,
 
     // Final state (src/celeritas/em/interactor/detail/IoniFinalStateHelper.hh)
     real_type const momentum
-        = std::sqrt(secondary_energy * (secondary_energy + 2 * electron_mass));
-    real_type const costheta = secondary_energy
-                               * (inc_energy + electron_mass + electron_mass)
-                               / (momentum * inc_momentum);
+        = gbx::sqrt(secondary_energy * (secondary_energy + 2 * electron_mass));
+    real_type const costheta
+        = div(secondary_energy * (inc_energy + electron_mass + electron_mass),
+              momentum * inc_momentum);
     electron->energy = secondary_energy;
     electron->direction = sample_exiting_direction<real_type>(costheta, inc_dir, rng);
     electron->particle_id = p.electron_id;
@@ -855,9 +854,9 @@ GBX_FUNCTION Interaction interact_eplusgg(ParamsData const& p,
     else
     {
         constexpr real_type half = 0.5;
-        real_type const tau = inc_energy / electron_mass;
+        real_type const tau = div(inc_energy, electron_mass);
         real_type const tau2 = tau + 2;
-        real_type const sqgrate = std::sqrt(tau / tau2) * half;
+        real_type const sqgrate = gbx::sqrt(div(tau, tau2)) * half;
         ReciprocalDistribution<real_type> sample_eps(half - sqgrate,
                                                      half + sqgrate);
         real_type epsil;
@@ -865,11 +864,11 @@ GBX_FUNCTION Interaction interact_eplusgg(ParamsData const& p,
         {
             epsil = sample_eps(rng);
         } while (sample_bernoulli<real_type>(
-            epsil - (2 * (tau + 1) * epsil - 1) / (epsil * ipow<2>(tau2)), rng));
-        real_type const cost = (epsil * tau2 - 1) / (epsil * std::sqrt(tau * tau2));
+            epsil - div(2 * (tau + 1) * epsil - 1, epsil * ipow<2>(tau2)), rng));
+        real_type const cost = div(epsil * tau2 - 1, epsil * gbx::sqrt(tau * tau2));
         real_type const total_energy = inc_energy + 2 * electron_mass;
         real_type const gamma_energy = epsil * total_energy;
-        real_type const eplus_moment = std::sqrt(inc_energy * total_energy);
+        real_type const eplus_moment = gbx::sqrt(inc_energy * total_energy);
         secondaries[0].energy = gamma_energy;
         secondaries[0].direction
             = sample_exiting_direction<real_type>(cost, inc_dir, rng);

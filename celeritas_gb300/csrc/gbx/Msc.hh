@@ -54,15 +54,15 @@ class MscHelper
     GBX_FORCEINLINE real_type calc_msc_mfp(real_type energy) const
     {
         real_type xsec
-            = calc_grid_xs(p_, *xs_, energy, phys_.log_energy(energy)) / ipow<2>(energy);
+            = div(calc_grid_xs(p_, *xs_, energy, phys_.log_energy(energy)), ipow<2>(energy));
         if constexpr (sizeof(real_type) < sizeof(double))
         {
             // FP32: in a near-vacuum the cross section underflows to zero;
             // a finite mean free path far beyond any step keeps the
             // path conversions finite (tau = step / lambda stays ~0)
-            return min_of(1 / xsec, real_type(1e20));
+            return min_of(div(1, xsec), real_type(1e20));
         }
-        return 1 / xsec;
+        return div(1, xsec);
     }
 
     GBX_FORCEINLINE real_type calc_inverse_range(real_type step) const
@@ -128,7 +128,7 @@ GBX_FUNCTION GeoPath msc_true_to_geo(ParamsData const& p,
     }
     else if (tstep < range * msc::dtrl)
     {
-        result.step = -lambda * libm::expm1(-tstep / lambda);
+        result.step = -lambda * libm::expm1(div(-tstep, lambda));
     }
     else
     {
@@ -136,7 +136,7 @@ GBX_FUNCTION GeoPath msc_true_to_geo(ParamsData const& p,
         real_type const mass = p.particles[p.electron_id].mass;
         if (energy < mass || tstep == range)
         {
-            result.alpha = 1 / range;
+            result.alpha = div(1, range);
             mfp_slope = max_of<real_type>(1 - result.alpha * tstep, 0);
         }
         else
@@ -144,12 +144,12 @@ GBX_FUNCTION GeoPath msc_true_to_geo(ParamsData const& p,
             real_type rfinal = range - tstep;
             real_type endpoint_energy = helper.calc_inverse_range(rfinal);
             real_type lambda1 = helper.calc_msc_mfp(endpoint_energy);
-            result.alpha = (lambda - lambda1) / (lambda * tstep);
-            mfp_slope = lambda1 / lambda;
+            result.alpha = div(lambda - lambda1, lambda * tstep);
+            mfp_slope = div(lambda1, lambda);
         }
-        real_type w = 1 + 1 / (result.alpha * lambda);
-        result.step = (1 - real_type(libm::exp(w * libm::log(mfp_slope))))
-                      / (result.alpha * w);
+        real_type w = 1 + div(1, result.alpha * lambda);
+        result.step = div(1 - real_type(libm::exp(w * libm::log(mfp_slope))),
+                          result.alpha * w);
     }
     result.step = min_of(result.step, tstep);
     return result;
@@ -169,7 +169,7 @@ GBX_FUNCTION real_type msc_geo_to_true(real_type true_step,
     real_type tstep;
     if (alpha == msc::small_step_alpha)
     {
-        tstep = -lambda * libm::log1p(-gstep / lambda);
+        tstep = -lambda * libm::log1p(div(-gstep, lambda));
         if (tstep < msc::min_step)
         {
             tstep = gstep;
@@ -177,11 +177,11 @@ GBX_FUNCTION real_type msc_geo_to_true(real_type true_step,
     }
     else
     {
-        real_type w = 1 + 1 / (alpha * lambda);
+        real_type w = 1 + div(1, alpha * lambda);
         real_type x = alpha * w * gstep;
         x = min_of(x, real_type(1));
-        real_type temp = 1 - libm::exp((1 / w) * libm::log(1 - x));
-        real_type result = temp / alpha;
+        real_type temp = 1 - libm::exp(div(1, w) * libm::log(1 - x));
+        real_type result = div(temp, alpha);
         tstep = min_of(result, range);
     }
     // clamp(tstep, gstep, true_step)
@@ -192,7 +192,7 @@ GBX_FORCEINLINE real_type msc_displacement(real_type geom_path, real_type true_p
 {
     real_type rmax2 = (true_path - geom_path) * (true_path + geom_path);
     constexpr real_type mean_radius_frac{0.73};
-    return mean_radius_frac * std::sqrt(rmax2);
+    return mean_radius_frac * gbx::sqrt(rmax2);
 }
 
 //! Whether msc applies to this track for this step (UrbanMsc::is_applicable)
@@ -278,18 +278,18 @@ GBX_FUNCTION double msc_limit_step(ParamsData const& p,
                 if (helper.msc_mfp() > lambda_limit)
                 {
                     real_type c = 0.75;
-                    range_factor *= c + (1 - c) * helper.msc_mfp() / lambda_limit;
+                    range_factor *= c + div((1 - c) * helper.msc_mfp(), lambda_limit);
                 }
                 // calc_limit_min
                 UrbanMscMaterialRecord const& md = p.msc.material[mid];
                 real_type const cq[3] = {2, real_type(md.stepmin_coeff[0]),
                                          real_type(md.stepmin_coeff[1])};
-                real_type xm = helper.msc_mfp() / poly_eval<2>(cq, energy);
+                real_type xm = div(helper.msc_mfp(), poly_eval<2>(cq, energy));
                 xm *= helper.scaled_zeff();
                 if (energy < msc::min_scaling_energy)
                 {
                     xm *= (real_type(0.5)
-                           + real_type(0.5) * energy / msc::min_scaling_energy);
+                           + div(real_type(0.5) * energy, msc::min_scaling_energy));
                 }
                 real_type limit_min = max_of<real_type>(xm, msc::limit_min_fix);
                 s.msc_range_init[slot] = range_init;
@@ -354,14 +354,14 @@ GBX_FORCEINLINE real_type urban_positron_correction(real_type zeff, real_type y)
     real_type const c_m[3]
         = {real_type(1.41125), real_type(-1.86427e-2), real_type(1.84035e-4)};
     real_type const a = poly_eval<1>(c_a, zeff);
-    real_type const b = poly_eval<2>(c_b, 1 / zeff);
+    real_type const b = poly_eval<2>(c_b, div(1, zeff));
     real_type const c = poly_eval<1>(c_c, zeff);
     real_type const d = real_type(1.21e-3) * zeff;
     real_type const mult = poly_eval<2>(c_m, zeff);
     constexpr real_type xl = 0.6;
     constexpr real_type xh = 0.9;
     constexpr real_type e = 113;
-    real_type x = std::sqrt(y * (y + 2) / ipow<2>(y + 1));
+    real_type x = gbx::sqrt(div(y * (y + 2), ipow<2>(y + 1)));
     real_type corr;
     if (x < xl)
     {
@@ -375,7 +375,7 @@ GBX_FORCEINLINE real_type urban_positron_correction(real_type zeff, real_type y)
     {
         real_type yl = a * (1 - libm::exp(-b * xl));
         real_type yh = c + d * libm::exp(e * (xh - 1));
-        real_type y0 = (yh - yl) / (xh - xl);
+        real_type y0 = div(yh - yl, xh - xl);
         real_type y1 = yl - y0 * xl;
         corr = y0 * x + y1;
     }
@@ -465,36 +465,36 @@ GBX_FUNCTION void msc_apply_step(ParamsData const& p,
         if (std::fabs(lambda - lambda_end) < lambda * real_type(0.01))
             denom = helper.msc_mfp();
         else
-            denom = (lambda - lambda_end) / libm::log(lambda / lambda_end);
-        tau = true_path / denom;
+            denom = div(lambda - lambda_end, libm::log(div(lambda, lambda_end)));
+        tau = div(true_path, denom);
         if (tau < msc::tau_big)
         {
             xmean = libm::exp(-tau);
-            x2mean = (1 + 2 * libm::exp(real_type(-2.5) * tau)) / 3;
+            x2mean = div(1 + 2 * libm::exp(real_type(-2.5) * tau), 3);
             if (limit_min == 0)
                 limit_min = msc::limit_min;
             limit_min = min_of(limit_min, real_type(p.msc.lambda_limit));
             // compute_theta0
             real_type const mass = p.particles[p.electron_id].mass;
             real_type tp = max_of(limit_min, true_path);
-            real_type y = tp / real_type(mat.rad_length);
+            real_type y = div(tp, real_type(mat.rad_length));
             if (is_positron)
             {
                 y *= urban_positron_correction(
-                    real_type(mat.zeff), std::sqrt(inc_energy * end_energy) / mass);
+                    real_type(mat.zeff), div(gbx::sqrt(inc_energy * end_energy), mass));
             }
-            real_type invbetacp = std::sqrt(
-                (inc_energy + mass) * (end_energy + mass)
-                / (inc_energy * (inc_energy + 2 * mass) * end_energy
-                   * (end_energy + 2 * mass)));
+            real_type invbetacp
+                = gbx::sqrt(div((inc_energy + mass) * (end_energy + mass),
+                                inc_energy * (inc_energy + 2 * mass) * end_energy
+                                    * (end_energy + 2 * mass)));
             constexpr real_type c_highland = 13.6;
-            real_type th = c_highland * std::sqrt(y) * invbetacp;
+            real_type th = c_highland * gbx::sqrt(y) * invbetacp;
             real_type const tc[2] = {real_type(md.theta_coeff[0]),
                                      real_type(md.theta_coeff[1])};
             th *= poly_eval<1>(tc, libm::log(y));
             if (true_path < limit_min)
             {
-                th *= std::sqrt(true_path / limit_min);
+                th *= gbx::sqrt(div(true_path, limit_min));
             }
             theta0 = max_of<real_type>(th, 0);
             if (theta0 < real_type(1e-8))
@@ -510,15 +510,15 @@ GBX_FUNCTION void msc_apply_step(ParamsData const& p,
         return;
 
     auto simple_scattering = [&]() -> real_type {
-        real_type a = (2 * xmean + 9 * x2mean - 3) / (2 * xmean - 3 * x2mean + 1);
-        real_type p_pow = (a + 2) * xmean / a;
+        real_type a = div(2 * xmean + 9 * x2mean - 3, 2 * xmean - 3 * x2mean + 1);
+        real_type p_pow = div((a + 2) * xmean, a);
         real_type result{};
         do
         {
             real_type rdm = generate_canonical<real_type>(rng);
             result = 2
                          * (sample_bernoulli<real_type>(p_pow, rng)
-                                ? real_type(libm::exp((1 / (a + 1)) * libm::log(rdm)))
+                                ? real_type(libm::exp(div(1, a + 1) * libm::log(rdm)))
                                 : rdm)
                      - 1;
         } while (std::fabs(result) > 1);
@@ -541,9 +541,9 @@ GBX_FUNCTION void msc_apply_step(ParamsData const& p,
     else
     {
         // sample_cos_theta
-        real_type maxtau = true_path < limit_min ? limit_min / helper.msc_mfp() : tau;
+        real_type maxtau = true_path < limit_min ? div(limit_min, helper.msc_mfp()) : tau;
         real_type u = libm::exp((1 / real_type(6)) * libm::log(maxtau));
-        real_type radlen_mfp = true_path / (tau * real_type(mat.rad_length));
+        real_type radlen_mfp = div(true_path, tau * real_type(mat.rad_length));
         real_type const tq[3] = {real_type(md.tail_coeff[0]),
                                  real_type(md.tail_coeff[1]),
                                  real_type(md.tail_coeff[2])};
@@ -552,7 +552,7 @@ GBX_FUNCTION void msc_apply_step(ParamsData const& p,
         xsi = max_of(xsi, real_type(1.9));
         real_type ea = libm::exp(-xsi);
         real_type x = ipow<2>(2 * libm::sin(real_type(0.5) * theta0));
-        real_type xmean_1 = 1 - x * (1 + (xsi * ea) / (1 - ea));
+        real_type xmean_1 = 1 - x * (1 + div(xsi * ea, 1 - ea));
         if (xmean_1 <= real_type(0.999) * xmean)
         {
             costheta = simple_scattering();
@@ -567,12 +567,12 @@ GBX_FUNCTION void msc_apply_step(ParamsData const& p,
             else
                 c = xsi;
             real_type b1 = 2 + (c - xsi) * x;
-            real_type d = libm::exp((c - 1) * libm::log(c * x / b1));
+            real_type d = libm::exp((c - 1) * libm::log(div(c * x, b1)));
             real_type x0 = 1 - xsi * x;
-            real_type xmean_2 = (x0 + d - (c * x - b1 * d) / (c - 2)) / (1 - d);
-            real_type f2x0 = (c - 1) / (c * (1 - d));
-            real_type prob = f2x0 / (ea / (1 - ea) + f2x0);
-            real_type qprob = xmean / (prob * xmean_1 + (1 - prob) * xmean_2);
+            real_type xmean_2 = div(x0 + d - div(c * x - b1 * d, c - 2), 1 - d);
+            real_type f2x0 = div(c - 1, c * (1 - d));
+            real_type prob = div(f2x0, div(ea, 1 - ea) + f2x0);
+            real_type qprob = div(xmean, prob * xmean_1 + (1 - prob) * xmean_2);
             if (generate_canonical<real_type>(rng) >= qprob)
             {
                 costheta = UniformRealDistribution<real_type>(-1, 1)(rng);
@@ -587,7 +587,7 @@ GBX_FUNCTION void msc_apply_step(ParamsData const& p,
                 real_type var = (1 - d) * generate_canonical<real_type>(rng);
                 if (var < real_type(0.01) * d)
                 {
-                    var /= (d * (c - 1));
+                    var = div(var, d * (c - 1));
                     costheta = -1
                                + var * (1 - real_type(0.5) * var * c)
                                      * (2 + (c - xsi) * x);
@@ -598,7 +598,7 @@ GBX_FUNCTION void msc_apply_step(ParamsData const& p,
                                    * (c - xsi
                                       - c
                                             * real_type(libm::exp(
-                                                (-1 / (c - 1)) * libm::log(var + d))))
+                                                div(-1, c - 1) * libm::log(var + d))))
                                + 1;
                 }
             }
@@ -617,8 +617,8 @@ GBX_FUNCTION void msc_apply_step(ParamsData const& p,
             // sample_displacement_dir
             constexpr real_type cbeta = 2.160;
             constexpr real_type cbeta1 = 0.9988703417569197;
-            real_type psi = -libm::log(1 - generate_canonical<real_type>(rng) * cbeta1)
-                            / cbeta;
+            real_type psi = div(
+                -libm::log(1 - generate_canonical<real_type>(rng) * cbeta1), cbeta);
             real_type dphi = phi;
             dphi += sample_bernoulli<real_type>(real_type(0.5), rng) ? psi : -psi;
             RVec3 dd{libm::cos(dphi), libm::sin(dphi), 0};

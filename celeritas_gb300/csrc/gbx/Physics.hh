@@ -24,7 +24,7 @@ namespace gbx
 template<class T>
 GBX_FORCEINLINE T interp_linear(T x0, T y0, T x1, T y1, T x)
 {
-    T slope = (-y0 + y1) / (-x0 + x1);
+    T slope = div(-y0 + y1, -x0 + x1);
     return gbx_fma(slope, (-x0 + x), y0);
 }
 
@@ -67,23 +67,23 @@ GBX_FORCEINLINE real_type calc_grid_xs(ParamsData const& p,
     auto extrapolated = [&](size_type idx) {
         real_type result = values[idx];
         if (idx >= g.prime_index)
-            result /= energy;
+            result = div(result, energy);
         return result;
     };
     if (loge <= g.log_front)
         return extrapolated(0);
     if (loge >= g.log_back)
         return extrapolated(g.size - 1);
-    size_type lower = static_cast<size_type>((loge - g.log_front) / g.log_delta);
+    size_type lower = static_cast<size_type>(div(loge - g.log_front, g.log_delta));
     lower = min_of(lower, g.size - 2);
     real_type upper_energy = energies[lower + 1];
     real_type upper_xs = values[lower + 1];
     if (lower + 1 == g.prime_index)
-        upper_xs /= upper_energy;
+        upper_xs = div(upper_xs, upper_energy);
     real_type result = interp_linear<real_type>(
         energies[lower], values[lower], upper_energy, upper_xs, energy);
     if (lower >= g.prime_index)
-        result /= energy;
+        result = div(result, energy);
     return result;
 }
 
@@ -112,7 +112,7 @@ GBX_FORCEINLINE real_type calc_range(ParamsData const& p,
     }
     if (loge >= g.log_back)
         return values[g.size - 1];
-    size_type idx = static_cast<size_type>((loge - g.log_front) / g.log_delta);
+    size_type idx = static_cast<size_type>(div(loge - g.log_front, g.log_delta));
     idx = min_of(idx, g.size - 2);
     return interp_linear<real_type>(
         energies[idx], values[idx], energies[idx + 1], values[idx + 1], energy);
@@ -135,7 +135,7 @@ GBX_FORCEINLINE real_type calc_inverse_range(ParamsData const& p,
     real_type const* energies = p.reals + g.energy;
     if (range < values[0])
     {
-        return energies[0] * ipow<2>(range / values[0]);
+        return energies[0] * ipow<2>(div(range, values[0]));
     }
     if (range >= values[g.size - 1])
     {
@@ -175,7 +175,7 @@ GBX_FORCEINLINE real_type livermore_pe_micro_xs(ParamsData const& p,
     LivermoreShell const* shells = p.livermore_shells + el.shells;
     real_type energy = max_of(inc_energy,
                               real_type(shells[el.num_shells - 1].binding_energy));
-    real_type inv_energy = real_type(1.) / energy;
+    real_type inv_energy = div(real_type(1.), energy);
     real_type result = 0.;
     if (energy >= el.thresh_lo)
     {
@@ -220,15 +220,15 @@ GBX_FORCEINLINE real_type eplusgg_macro_xs(ParamsData const& p,
                                            real_type energy)
 {
     real_type const electron_mass = p.particles[p.electron_id].mass;
-    real_type const gamma = max_of(energy, real_type(1e-6)) / electron_mass;
-    real_type const sqrt_gg2 = std::sqrt(gamma * (gamma + 2));
+    real_type const gamma = div(max_of(energy, real_type(1e-6)), electron_mass);
+    real_type const sqrt_gg2 = gbx::sqrt(gamma * (gamma + 2));
     real_type const quad[3] = {1, 4, 1};
     real_type result
-        = real_type(constants::pi) * ipow<2>(real_type(constants::r_electron))
-          * real_type(mat.electron_density)
-          * (poly_eval<2>(quad, gamma + 1) * libm::log(gamma + 1 + sqrt_gg2)
-             - (gamma + 4) * sqrt_gg2)
-          / (gamma * ipow<2>(gamma + 2));
+        = div(real_type(constants::pi) * ipow<2>(real_type(constants::r_electron))
+                  * real_type(mat.electron_density)
+                  * (poly_eval<2>(quad, gamma + 1) * libm::log(gamma + 1 + sqrt_gg2)
+                     - (gamma + 4) * sqrt_gg2),
+              gamma * ipow<2>(gamma + 2));
     return result;
 }
 
@@ -407,7 +407,7 @@ class PhysicsTrack
         if (range < rho * (1 + sqrt_tol))
             return range;
         real_type const alpha = p_.max_step_over_range;
-        return alpha * range + rho * (1 - alpha) * (2 - rho / range);
+        return alpha * range + rho * (1 - alpha) * (2 - div(rho, range));
     }
 
   private:
@@ -429,7 +429,7 @@ class PhysicsTrack
 //---------------------------------------------------------------------------//
 GBX_FORCEINLINE real_type beta_sq(real_type mass, real_type energy)
 {
-    real_type inv_gamma = mass / (energy + mass);
+    real_type inv_gamma = div(mass, energy + mass);
     return 1 - ipow<2>(inv_gamma);
 }
 GBX_FORCEINLINE real_type momentum_sq(real_type mass, real_type energy)
@@ -477,9 +477,9 @@ GBX_FUNCTION real_type sample_urban_eloss(UrbanFluctRecord const& params,
     constexpr real_type fwhm_min_energy = 1e-3;
 
     real_type const loss_scaling
-        = real_type(0.5) * min_of(fwhm_min_energy / max_energy, real_type(1))
+        = real_type(0.5) * min_of(div(fwhm_min_energy, max_energy), real_type(1))
           + real_type(1);
-    real_type const mean_loss = unscaled_mean_loss / loss_scaling;
+    real_type const mean_loss = div(unscaled_mean_loss, loss_scaling);
 
     real_type binding_energy[2] = {real_type(params.binding_energy[0]),
                                    real_type(params.binding_energy[1])};
@@ -492,32 +492,31 @@ GBX_FUNCTION real_type sample_urban_eloss(UrbanFluctRecord const& params,
         {
             if (w > real_type(params.log_binding_energy[1]))
             {
-                real_type const c = mean_loss * (1 - rate) / (w - w_0);
+                real_type const c = div(mean_loss * (1 - rate), w - w_0);
                 for (int i = 0; i < 2; ++i)
                 {
-                    xs_exc[i] = c * real_type(params.oscillator_strength[i])
-                                * (w - real_type(params.log_binding_energy[i]))
-                                / real_type(params.binding_energy[i]);
+                    xs_exc[i] = div(c * real_type(params.oscillator_strength[i])
+                                        * (w - real_type(params.log_binding_energy[i])),
+                                    real_type(params.binding_energy[i]));
                 }
             }
             else
             {
-                xs_exc[0] = mean_loss * (1 - rate)
-                            / real_type(params.binding_energy[0]);
+                xs_exc[0] = div(mean_loss * (1 - rate), real_type(params.binding_energy[0]));
             }
             real_type scaling = 4;
             if (xs_exc[0] < exc_thresh)
             {
                 scaling = real_type(0.5)
                           + (scaling - real_type(0.5))
-                                * std::sqrt(xs_exc[0] / exc_thresh);
+                                * gbx::sqrt(div(xs_exc[0], exc_thresh));
             }
             binding_energy[0] *= scaling;
-            xs_exc[0] /= scaling;
+            xs_exc[0] = div(xs_exc[0], scaling);
         }
     }
-    real_type xs_ion = mean_loss * (max_energy - e_0)
-                       / (max_energy * e_0 * libm::log(max_energy / e_0));
+    real_type xs_ion = div(mean_loss * (max_energy - e_0),
+                           max_energy * e_0 * libm::log(div(max_energy, e_0)));
     if (xs_exc[0] + xs_exc[1] > 0)
     {
         xs_ion *= rate;
@@ -548,36 +547,36 @@ GBX_FUNCTION real_type sample_urban_eloss(UrbanFluctRecord const& params,
         }
         if (variance > 0)
         {
-            exc_result += sample_fast_urban(mean, std::sqrt(variance), rng);
+            exc_result += sample_fast_urban(mean, gbx::sqrt(variance), rng);
         }
     }
 
     // Ionization loss
     real_type ion_result = 0;
     {
-        real_type const energy_ratio = max_energy / e_0;
+        real_type const energy_ratio = div(max_energy, e_0);
         real_type alpha = 1;
         real_type mean_num_coll = 0;
         if (xs_ion > max_collisions)
         {
-            alpha = (xs_ion + max_collisions) * energy_ratio
-                    / (max_collisions * energy_ratio + xs_ion);
-            real_type const mean_loss_coll = alpha * libm::log(alpha) / (alpha - 1);
-            mean_num_coll = xs_ion * energy_ratio * (alpha - 1)
-                            / ((energy_ratio - 1) * alpha);
+            alpha = div((xs_ion + max_collisions) * energy_ratio,
+                        max_collisions * energy_ratio + xs_ion);
+            real_type const mean_loss_coll = div(alpha * libm::log(alpha), alpha - 1);
+            mean_num_coll
+                = div(xs_ion * energy_ratio * (alpha - 1), (energy_ratio - 1) * alpha);
             real_type const mean = mean_num_coll * mean_loss_coll * e_0;
             real_type const stddev
-                = e_0 * std::sqrt(xs_ion * (alpha - ipow<2>(mean_loss_coll)));
+                = e_0 * gbx::sqrt(xs_ion * (alpha - ipow<2>(mean_loss_coll)));
             ion_result += sample_fast_urban(mean, stddev, rng);
         }
         if (xs_ion > 0 && energy_ratio > alpha)
         {
             real_type const lambda = xs_ion - mean_num_coll;
             UniformRealDistribution<real_type> sample_fraction(
-                alpha / energy_ratio, 1);
+                div(alpha, energy_ratio), 1);
             for (auto n = sample_poisson<real_type>(lambda, rng); n > 0; --n)
             {
-                ion_result += alpha * e_0 / sample_fraction(rng);
+                ion_result += div(alpha * e_0, sample_fraction(rng));
             }
         }
     }

@@ -258,7 +258,7 @@ GBX_FORCEINLINE bool sample_bernoulli(T p_true, G& rng)
 GBX_FORCEINLINE real_type bernoulli_p(real_type scaled_true,
                                       real_type scaled_false)
 {
-    return scaled_true / (scaled_true + scaled_false);
+    return div(scaled_true, scaled_true + scaled_false);
 }
 
 //! Reciprocal (log-uniform) distribution on [a, b]
@@ -268,7 +268,7 @@ struct ReciprocalDistribution
     T a;
     T logratio;
     GBX_FORCEINLINE ReciprocalDistribution(T lo, T hi)
-        : a(lo), logratio(libm::log((1 / lo) * hi))
+        : a(lo), logratio(libm::log(div(1, lo) * hi))
     {
     }
     template<class G>
@@ -304,7 +304,7 @@ class NormalDistribution
         }
         constexpr T twopi = static_cast<T>(2 * constants::pi);
         T theta = twopi * generate_canonical<T>(rng);
-        T r = std::sqrt(-2 * libm::log(generate_canonical<T>(rng)));
+        T r = gbx::sqrt(-2 * libm::log(generate_canonical<T>(rng)));
         spare_ = r * libm::cos(theta);
         has_spare_ = true;
         return gbx_fma(r * libm::sin(theta), stddev_, mean_);
@@ -332,7 +332,7 @@ GBX_FORCEINLINE unsigned int sample_poisson(T lambda, G& rng)
         } while (p > 1);
         return static_cast<unsigned int>(k - 1);
     }
-    NormalDistribution<T> sample_normal(lambda, std::sqrt(lambda));
+    NormalDistribution<T> sample_normal(lambda, gbx::sqrt(lambda));
     return static_cast<unsigned int>(sample_normal(rng) + T(0.5));
 }
 

@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstdint>
 
+#include "Fp64.hh"
 #include "Libm.hh"
 #include "Macros.hh"
 
@@ -120,13 +121,13 @@ GBX_FORCEINLINE T dot_product(Vec3<T> const& a, Vec3<T> const& b)
 template<class T>
 GBX_FORCEINLINE T norm(Vec3<T> const& v)
 {
-    return std::sqrt(dot_product(v, v));
+    return gbx::sqrt(dot_product(v, v));
 }
 
 template<class T>
 GBX_FORCEINLINE Vec3<T> make_unit_vector(Vec3<T> const& v)
 {
-    T const scale = T(1) / norm(v);
+    T const scale = div(T(1), norm(v));
     return {v.x * scale, v.y * scale, v.z * scale};
 }
 
@@ -161,7 +162,7 @@ GBX_FORCEINLINE void axpy(T a, Vec3<T> const& x, Vec3<T>* y)
 template<class T>
 GBX_FORCEINLINE Vec3<T> from_spherical(T costheta, T phi)
 {
-    T const sintheta = std::sqrt(1 - costheta * costheta);
+    T const sintheta = gbx::sqrt(1 - costheta * costheta);
     return {sintheta * libm::cos(phi), sintheta * libm::sin(phi), costheta};
 }
 
@@ -171,19 +172,19 @@ template<class T>
 GBX_FORCEINLINE Vec3<T> rotate(Vec3<T> const& dir, Vec3<T> const& rot)
 {
     constexpr T min_accurate_sintheta = sizeof(T) == 8 ? T(0.005) : T(0.07);
-    T sintheta = std::sqrt(1 - ipow<2>(rot.z));
+    T sintheta = gbx::sqrt(1 - ipow<2>(rot.z));
     T cosphi;
     T sinphi;
     if (sintheta >= min_accurate_sintheta)
     {
-        T const inv_sintheta = 1 / (sintheta);
+        T const inv_sintheta = div(1, sintheta);
         cosphi = rot.x * inv_sintheta;
         sinphi = rot.y * inv_sintheta;
     }
     else if (sintheta > 0)
     {
-        cosphi = rot.x / std::sqrt(ipow<2>(rot.x) + ipow<2>(rot.y));
-        sinphi = std::sqrt(1 - ipow<2>(cosphi));
+        cosphi = div(rot.x, gbx::sqrt(ipow<2>(rot.x) + ipow<2>(rot.y)));
+        sinphi = gbx::sqrt(1 - ipow<2>(cosphi));
     }
     else
     {
