@@ -31,6 +31,11 @@
 //   double-double from exp(log(x)/3), then the cubes of the two rounding
 //   midpoints against x), with rounding tests where a fast form is used.
 //
+// The device evaluates exp, log, sin, cos, expm1 and log1p in fixed point first
+// (LibmInt.hh: the same correctly rounded doubles for a fraction of the cost
+// there) and comes back to these methods for the few arguments that leaves
+// undecided; the host always uses them, so that either checks the other.
+//
 // "Correctly rounded" holds except possibly for the few inputs whose exact
 // result lies within about 2^-100 (relative) of a rounding midpoint, which
 // the accurate paths cannot separate; sin and cos additionally need
@@ -46,6 +51,7 @@
 #include <cstdint>
 #include <cstring>
 
+#include "LibmInt.hh"
 #include "LibmTables.hh"
 #include "Macros.hh"
 
@@ -319,13 +325,11 @@ GBX_NOINLINE double exp_accurate(double x)
 }
 }  // namespace detail
 
-//! exp(x), correctly rounded
-GBX_FORCEINLINE double exp(double x)
+namespace detail
 {
-#if defined(GBX_SYSTEM_LIBM)
-    return std::exp(x);
-#else
-    using namespace detail;
+//! exp(x) in double-doubles
+GBX_NOINLINE double exp_dd_rounded(double x)
+{
     if (!(x == x))
         return x + x;
     if (x > 0x1.62e42fefa39efp+9)
@@ -342,6 +346,31 @@ GBX_FORCEINLINE double exp(double x)
     if (ok)
         return y;
     return exp_accurate(x);
+}
+}  // namespace detail
+
+// The device's functions evaluate in fixed point first (LibmInt.hh) and return
+// here for the arguments that leaves undecided; they are functions of their own,
+// one copy of the code for all call sites, as Fp64.hh's operations are.
+#if defined(__CUDA_ARCH__)
+#    define GBX_LIBM_FIXED(CALL)           \
+        {                                  \
+            std::uint64_t result;          \
+            if (CALL)                      \
+                return detail::from_bits(result); \
+        }
+#else
+#    define GBX_LIBM_FIXED(CALL)
+#endif
+
+//! exp(x), correctly rounded
+GBX_NOINLINE double exp(double x)
+{
+#if defined(GBX_SYSTEM_LIBM)
+    return std::exp(x);
+#else
+    GBX_LIBM_FIXED(fixed::exp(detail::bits(x), &result));
+    return detail::exp_dd_rounded(x);
 #endif
 }
 
@@ -457,13 +486,11 @@ GBX_NOINLINE DD log_accurate(LogReduced const& red)
 }
 }  // namespace detail
 
-//! log(x), correctly rounded
-GBX_FORCEINLINE double log(double x)
+namespace detail
 {
-#if defined(GBX_SYSTEM_LIBM)
-    return std::log(x);
-#else
-    using namespace detail;
+//! log(x) in double-doubles
+GBX_NOINLINE double log_dd_rounded(double x)
+{
     if (!(x > 0) || x > 0x1.fffffffffffffp+1023)
     {
         if (x == 0)
@@ -480,6 +507,17 @@ GBX_FORCEINLINE double log(double x)
         return v.hi + v.lo;
     v = log_accurate(red);
     return v.hi + v.lo;
+}
+}  // namespace detail
+
+//! log(x), correctly rounded
+GBX_NOINLINE double log(double x)
+{
+#if defined(GBX_SYSTEM_LIBM)
+    return std::log(x);
+#else
+    GBX_LIBM_FIXED(fixed::log(detail::bits(x), &result));
+    return detail::log_dd_rounded(x);
 #endif
 }
 
@@ -581,7 +619,7 @@ GBX_NOINLINE DD trig_accurate(DD r, bool odd)
 }
 
 //! sin (quadrant offset 0) or cos (offset 1) of x, correctly rounded
-GBX_FORCEINLINE double sin_cos(double x, int offset)
+GBX_NOINLINE double sin_cos(double x, int offset)
 {
     int q;
     DD r = trig_reduce(x, &q);
@@ -609,6 +647,7 @@ GBX_NOINLINE double sin(double x)
 #if defined(GBX_SYSTEM_LIBM)
     return std::sin(x);
 #else
+    GBX_LIBM_FIXED(fixed::sin_cos(detail::bits(x), 0, &result));
     if (!(std::fabs(x) <= 0x1.fffffffffffffp+1023))
         return (x - x) / (x - x);
     if (std::fabs(x) < 0x1p-26)
@@ -623,6 +662,7 @@ GBX_NOINLINE double cos(double x)
 #if defined(GBX_SYSTEM_LIBM)
     return std::cos(x);
 #else
+    GBX_LIBM_FIXED(fixed::sin_cos(detail::bits(x), 1, &result));
     if (!(std::fabs(x) <= 0x1.fffffffffffffp+1023))
         return (x - x) / (x - x);
     if (std::fabs(x) < 0x1p-27)
@@ -692,6 +732,7 @@ GBX_NOINLINE double expm1(double x)
     return std::expm1(x);
 #else
     using namespace detail;
+    GBX_LIBM_FIXED(fixed::expm1(bits(x), &result));
     if (!(x == x))
         return x + x;
     if (x > 0x1.62e42fefa39efp+9)
@@ -715,6 +756,7 @@ GBX_NOINLINE double log1p(double x)
     return std::log1p(x);
 #else
     using namespace detail;
+    GBX_LIBM_FIXED(fixed::log1p(bits(x), &result));
     if (!(x > -1.0) || x > 0x1.fffffffffffffp+1023)
     {
         if (x == -1.0)

@@ -39,6 +39,12 @@ def dd(v):
     return hi, lo
 
 
+def i128(v, frac_bits: int) -> str:
+    """v times 2^frac_bits, nearest integer, as two 64-bit words."""
+    n = int(mpmath.nint(mpmath.mpf(v) * mpmath.mpf(2) ** frac_bits)) % (1 << 128)
+    return f"0x{n >> 64:016x}ull, 0x{n % (1 << 64):016x}ull"
+
+
 def h(x: float) -> str:
     return float(x).hex()
 
@@ -108,6 +114,36 @@ def main():
         hi, lo = dd(1 / mpmath.mpf(k)) if k else (0.0, 0.0)
         lines.append(f"    {h(hi)}, {h(lo)}")
     w(", \\\n".join(lines))
+    w("")
+    # Fixed-point tables of LibmInt.hh: 128-bit two's complement numbers as
+    # (high, low) 64-bit words
+    # log: interval j of [1, 2): C_j 2^-10 near the reciprocal of its center
+    # (exactly 1 and 1/2 in the first and last, so that log(x) near x = 1 is
+    # log1p of an exact argument), and -log(C_j 2^-10) times 2^117, less ln 2
+    # from j = 53 (m >= sqrt 2) on, where the exponent counts one more
+    w("#define GBX_LIBM_ILOG_TABLE \\")
+    lines = []
+    for j in range(N):
+        c = 1 + (mpmath.mpf(j) + mpmath.mpf(0.5)) / N
+        big_c = {0: 1024, N - 1: 512}.get(j, int(mpmath.nint(1024 / c)))
+        v = -mpmath.log(mpmath.mpf(big_c) / 1024) - (mpmath.log(2) if j >= 53 else 0)
+        lines.append(f"    {i128(v, 117)}, {big_c}u")
+    w(", \\\n".join(lines))
+    # exp: 2^(j/N) times 2^126
+    w("#define GBX_LIBM_IEXP_TABLE \\")
+    w(", \\\n".join(f"    {i128(mpmath.mpf(2) ** (mpmath.mpf(j) / N), 126)}" for j in range(N)))
+    for name, v, q in (("LN2_Q117", mpmath.log(2), 117), ("LN2_N_Q96", mpmath.log(2) / N, 96),
+                       ("PIO2_Q117", mpmath.pi / 2, 117)):
+        w(f"#define GBX_LIBM_{name} {i128(v, q)}")
+    # Taylor coefficients 1/k! times 2^q: 32-bit ones, then 64-bit ones
+    for name, ks, q, suffix in (("SIN_32", (19, 17, 15, 13), 64, "u"),
+                                ("SIN_64", (11, 9, 7, 5), 70, "ull"),
+                                ("COS_32", (20, 18, 16, 14), 64, "u"),
+                                ("COS_64", (12, 10, 8, 6, 4), 68, "ull"),
+                                ("EXPM1_32", (16, 15, 14, 13, 12, 11, 10), 52, ""),
+                                ("EXPM1_64", (9, 8, 7, 6, 5, 4, 3), 65, "ll")):
+        vals = [int(mpmath.nint(mpmath.mpf(2) ** q / mpmath.factorial(k))) for k in ks]
+        w(f"#define GBX_LIBM_{name} " + ", ".join(f"{v}{suffix}" for v in vals))
     w("")
     with open(os.path.join(HERE, "LibmTables.hh"), "w") as f:
         f.write("\n".join(out))

@@ -1,6 +1,8 @@
-// Device evaluation of gbx::div and gbx::sqrt, and host evaluation of their
-// significand routines with a perturbed reciprocal approximation.
+// Device evaluation of gbx::div and gbx::sqrt, host evaluation of their
+// significand routines with a perturbed reciprocal approximation, and host
+// evaluation of the fixed-point elementary functions.
 #include "../celeritas_gb300/csrc/gbx/Fp64.hh"
+#include "../celeritas_gb300/csrc/gbx/LibmInt.hh"
 
 namespace
 {
@@ -52,5 +54,25 @@ extern "C" void fp64_host(int op,
                                     | (static_cast<std::uint32_t>(a[i] >> (29 + odd)) & 0x7fffffu);
             y[i] = sqrt_significand(a[i], approx_rsqrt(f) + ulps);
         }
+    }
+}
+
+//! Bits of exp, log, sin, cos, expm1 or log1p (op 0-5) of x in fixed point;
+//! decided[i] is 0 where the function leaves the argument to double-doubles
+extern "C" void libm_fixed(int op,
+                           std::uint64_t const* x,
+                           std::uint64_t* y,
+                           unsigned char* decided,
+                           int n)
+{
+    namespace fixed = gbx::libm::fixed;
+    for (int i = 0; i < n; ++i)
+    {
+        decided[i] = op == 0   ? fixed::exp(x[i], y + i)
+                     : op == 1 ? fixed::log(x[i], y + i)
+                     : op == 2 ? fixed::sin_cos(x[i], 0, y + i)
+                     : op == 3 ? fixed::sin_cos(x[i], 1, y + i)
+                     : op == 4 ? fixed::expm1(x[i], y + i)
+                               : fixed::log1p(x[i], y + i);
     }
 }

@@ -1,12 +1,15 @@
-"""FP64 division and square root in integer arithmetic (gbx/Fp64.hh).
+"""FP64 division, square root (gbx/Fp64.hh) and elementary functions
+(gbx/LibmInt.hh) in integer arithmetic.
 
-Both are IEEE operations rounded to nearest even, so every result must equal
+The first two are IEEE operations rounded to nearest even, so every result must equal
 numpy's bit for bit. The operands cover the edges of the significand (all
 zeros, all ones, short and long runs of either), of the exponent range (the
 last normal and subnormal results, overflow) and the special values. The
 significand routines are also run on the host with the FP32 approximation
 they start from moved by 3 units in its last place, more than the 1 (rcp) and
-2 (rsqrt) that the hardware's instructions document.
+2 (rsqrt) that the hardware's instructions document. The elementary functions
+must return the correctly rounded value wherever they decide one, and decide
+all but a few in 2^9 arguments of the range they cover, to its edges.
 """
 
 import ctypes
@@ -63,6 +66,39 @@ def test_significands(lib, ulps):
     root = np.sqrt(x.astype(float) * 2.0**-52)
     expected = np.where(root < 2, fractions(root), np.uint64(1 << 53))
     np.testing.assert_array_equal(evaluate(1, x), expected)
+
+
+#: Range that the fixed-point functions cover, by magnitude and sign
+COVERED = {"exp": (2.0**-54, 708.3), "log": (2.3e-308, 1.7e308), "sin": (2.0**-26, 1023.9),
+           "cos": (2.0**-26, 1023.9), "expm1": (2.0**-54, 0.3499), "log1p": (2.0**-54, 0.9999)}
+
+
+@pytest.mark.parametrize("fn", list(COVERED))
+def test_fixed_point_functions(lib, built_port, fn):
+    import oracle
+
+    rng = np.random.default_rng(list(COVERED).index(fn))
+    lo, hi = COVERED[fn]
+    x = np.exp(rng.uniform(np.log(lo), np.log(hi), N))
+    x[:N // 2] = rng.uniform(lo, min(hi, 50.0), N // 2)
+    if fn == "log":
+        # Around 1, and the intervals that meet there
+        x[:N // 8] = 1 + rng.uniform(-1, 1, N // 8) * 2.0 ** rng.uniform(-40, -5, N // 8)
+    else:
+        x *= rng.choice([-1.0, 1.0], N)
+    if fn == "log1p":
+        x = np.where((x > 0) & (x >= 2.0**-7), -x, x)
+    y, decided = np.empty(N), np.empty(N, np.uint8)
+    lib.libm_fixed(list(COVERED).index(fn), x.ctypes.data_as(ctypes.c_void_p),
+                   y.ctypes.data_as(ctypes.c_void_p),
+                   decided.ctypes.data_as(ctypes.c_void_p), N)
+    ok = decided != 0
+    expected = oracle.port_libm(fn, x)
+    np.testing.assert_array_equal(y[ok].view(np.uint64), expected[ok].view(np.uint64))
+    # Tiny arguments (results near 1 or near the argument) are left out more
+    # often: a midpoint lies at half the last place of either
+    usual = (np.abs(x - (fn == "log")) > 2.0**-20)
+    assert np.mean(~ok[usual]) < 2.0**-8
 
 
 @pytest.mark.gpu
