@@ -882,7 +882,7 @@ __global__ GBX_ALONG_BOUNDS(Threads, 1) void along_charged_persistent_kernel(
     size_type const count = offsets ? offsets[end_bin] - first : s.size;
     unsigned int const lane = threadIdx.x & 31u;
     FieldOptions const& opt = p.field_options;
-    FieldPropagation fp(opt, UniformFieldEquation{});
+    FieldPropagation<false> fp(opt, UniformFieldEquation{});
     size_type slot = invalid_id;
     bool have = false;
     for (;;)

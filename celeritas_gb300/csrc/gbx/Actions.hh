@@ -275,11 +275,12 @@ GBX_FUNCTION bool along_prologue(ParamsData const& p,
 }
 
 //! Set up the uniform-field propagation of a charged slot over its step
+template<class Propagation>
 GBX_FUNCTION void field_setup(ParamsData const& p,
                               StateData const& s,
                               size_type slot,
                               GeoTrackView& geo,
-                              FieldPropagation* fp,
+                              Propagation* fp,
                               double start_safety)
 {
     size_type const pid = s.particle_id[slot];
@@ -449,7 +450,7 @@ GBX_FUNCTION void along_step_impl(ParamsData const& p, StateData const& s, size_
         if (charged && p.has_field)
         {
             FieldOptions const& opt = p.field_options;
-            FieldPropagation fp(opt, UniformFieldEquation{});
+            FieldPropagation<> fp(opt, UniformFieldEquation{});
             field_setup(p, s, slot, geo, &fp, start_safety);
             do
             {

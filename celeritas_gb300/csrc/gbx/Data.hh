@@ -339,6 +339,10 @@ struct FieldMapGrid
     double back;
     double delta;
     size_type size;
+    // The first three rounded to FP32 (mixed-precision stages)
+    float front_f;
+    float back_f;
+    float delta_f;
 };
 
 //! Field at a map node [native units]
@@ -387,6 +391,29 @@ struct FieldOptions
     static constexpr double initial_step_tol = 1e-6;
     static constexpr double dchord_tol = 1e-5 * constants::millimeter;
     static constexpr double min_chord_shrink = 0.5;
+
+    // FP32 forms of the above for the mixed-precision driver, set by derive():
+    //! Largest float not above delta_chord + dchord_tol: an FP32 chord
+    //! distance compares with it as with the sum
+    float chord_limit{};
+    //! From here on sqrt(delta_chord / distance) is below min_chord_shrink
+    float chord_far{};
+    //! 1 / epsilon_rel_max^2 as the sum of two floats
+    float inv_tolerance[2]{};
+
+    void derive()
+    {
+        double const limit = delta_chord + dchord_tol;
+        chord_limit = static_cast<float>(limit);
+        if (double(chord_limit) > limit)
+            chord_limit = std::nextafter(chord_limit, 0.0f);
+        chord_far = static_cast<float>(delta_chord * 4.01);
+        if (!(chord_far > chord_limit))
+            chord_far = chord_limit;
+        double const inv = 1 / (epsilon_rel_max * epsilon_rel_max);
+        inv_tolerance[0] = static_cast<float>(inv);
+        inv_tolerance[1] = static_cast<float>(inv - double(inv_tolerance[0]));
+    }
 
     //! Whether all values are valid (FieldDriverOptions::operator bool)
     bool valid() const

@@ -7,25 +7,19 @@
 // MagFieldEquation.hh, detail/FieldUtils.hh and the defaults of
 // FieldDriverOptions.hh:26-77.
 //
-// FP64 build: the whole integration is FP64, operation for operation as in
-// the reference. Mixed-precision build: the Runge-Kutta stages (field
-// evaluations and stage momenta) are FP32; the positions are accumulated in
-// FP64 from FP32 increments; the embedded error vector and the chord
-// distance are formed in FP32 from the FP32 stages, and the error norms, the
-// acceptance test, the step and the path length are FP64. The step-size
-// scale factor err^(-1/5) is FP32.
+// This file holds the FP64 build's driver, FP64 throughout, operation for
+// operation as in the reference, and the propagator of both builds; the
+// mixed-precision build's driver is in FieldMixed.hh.
 #pragma once
 
+#include <type_traits>
+
+#include "FieldMixed.hh"
+#include "FieldState.hh"
 #include "Geometry.hh"
 
 namespace gbx
 {
-struct OdeState
-{
-    Real3 pos;
-    Real3 mom;
-};
-
 GBX_FORCEINLINE void axpy(double a, OdeState const& x, OdeState* y)
 {
     axpy(a, x.pos, &y->pos);
@@ -76,70 +70,11 @@ GBX_FUNCTION Real3 rzmap_field(RZMapData const& m, Real3 const& pos)
     return value;
 }
 
-//! The R-Z map's field in FP32 (the mixed-precision stages): the same
-//! interpolation on the FP32 nodes at an FP32 position
-GBX_NOINLINE Vec3<float> rzmap_field_f(RZMapData const& m, Vec3<float> const& pos)
-{
-    Vec3<float> value{0, 0, 0};
-    float const r = gbx::sqrt(pos.x * pos.x + pos.y * pos.y);
-    if (!(pos.z >= float(m.z.front) && pos.z <= float(m.z.back) && r >= float(m.r.front)
-          && r <= float(m.r.back)))
-        return value;
-    auto locate = [](FieldMapGrid const& g, float v, size_type* index) {
-        float const u = div(v - float(g.front), float(g.delta));
-        size_type const i = min_of(static_cast<size_type>(u), g.size - 2);
-        *index = i;
-        return u - float(i);
-    };
-    size_type ir, iz;
-    float const fr = locate(m.r, r, &ir);
-    float const fz = locate(m.z, pos.z, &iz);
-    size_type const nr = m.r.size;
-    FieldMapElementF const* v = m.values_f;
-    float low = v[iz * nr + ir].value_z;
-    float high = v[(iz + 1) * nr + ir].value_z;
-    value.z = low + (high - low) * fz;
-    low = v[iz * nr + ir].value_r;
-    high = v[iz * nr + ir + 1].value_r;
-    float const tmp = (r != 0) ? div(low + (high - low) * fr, r) : low;
-    value.x = tmp * pos.x;
-    value.y = tmp * pos.y;
-    return value;
-}
-
-//! Equation of motion in a magnetic field: d(pos)/ds = p/|p|,
-//! d(mom)/ds = (q/|p|) p x B(pos) (MagFieldEquation). The field is uniform,
-//! or an R-Z map evaluated at the state's position when 'map' is set.
-struct UniformFieldEquation
-{
-    Real3 field;
-    double coeffi;
-    RZMapData const* map{nullptr};
-
-    GBX_FORCEINLINE OdeState operator()(OdeState const& y) const
-    {
-        double momentum_inv = div(1.0, gbx::sqrt(dot_product(y.mom, y.mom)));
-        OdeState result;
-        result.pos = {momentum_inv * y.mom.x,
-                      momentum_inv * y.mom.y,
-                      momentum_inv * y.mom.z};
-        double const scale = coeffi * momentum_inv;
-        Real3 c = cross_product(y.mom, map ? rzmap_field(*map, y.pos) : field);
-        result.mom = {scale * c.x, scale * c.y, scale * c.z};
-        return result;
-    }
-};
-
 struct FieldStepperResult
 {
-    OdeState mid_state;  //!< FP64 build only
+    OdeState mid_state;
     OdeState end_state;
-    OdeState err_state;  //!< FP64 build only
-    // Mixed-precision build only: the embedded error estimate and the chord
-    // distance, formed in FP32 from the FP32 stages
-    Vec3<float> err_pos_rate;  //!< position error / step = sum_i d_i k_pos_i
-    Vec3<float> err_mom;  //!< momentum error = step * sum_i d_i k_mom_i
-    float dchord;  //!< sagitta of the midpoint from the chord
+    OdeState err_state;
 };
 
 //! The field equation with its field source fixed at compile time, so that
@@ -255,176 +190,19 @@ GBX_FUNCTION FieldStepperResult dormand_prince_step_fp64(Equation const& rhs,
     return result;
 }
 
-
-//! Mixed-precision Dormand-Prince 5(4) step. The stages carry FP32 momenta,
-//! FP32 derivatives and, for a field map, FP32 position increments from the
-//! start at which the map is read in FP32; the end position is the FP64
-//! start plus an FP32 increment. The embedded error estimate (a weighted sum
-//! of the FP32 stage derivatives) and the chord distance (from the FP32
-//! increments to the end and to Shampine's midpoint) are formed in FP32:
-//! their inputs carry FP32 rounding, which FP64 arithmetic on them would not
-//! remove. The field driver takes the error norms and the acceptance test in FP64.
-GBX_FUNCTION FieldStepperResult dormand_prince_step_mixed(UniformFieldEquation const& rhs,
-                                                          double step,
-                                                          OdeState const& beg_state)
-{
-    using F = float;
-    using F3 = Vec3<float>;
-    // Butcher tableau of the FP64 stepper, rounded to FP32
-    constexpr F a11 = 0.2f;
-    constexpr F a21 = 0.075f, a22 = 0.225f;
-    constexpr F a31 = F(44. / 45), a32 = F(-56. / 15), a33 = F(32. / 9);
-    constexpr F a41 = F(19372. / 6561), a42 = F(-25360. / 2187),
-                a43 = F(64448. / 6561), a44 = F(-212. / 729);
-    constexpr F a51 = F(9017. / 3168), a52 = F(-355. / 33), a53 = F(46732. / 5247),
-                a54 = F(49. / 176), a55 = F(-5103. / 18656);
-    constexpr double b1 = 35. / 384, b3 = 500. / 1113, b4 = 125. / 192,
-                     b5 = -2187. / 6784, b6 = 11. / 84;
-    constexpr double d1 = b1 - 5179. / 57600, d3 = b3 - 7571. / 16695,
-                     d4 = b4 - 393. / 640, d5 = b5 + 92097. / 339200,
-                     d6 = b6 - 187. / 2100, d7 = -1. / 40;
-    constexpr F c1 = F(6025192743. / 30085553152.), c3 = F(51252292925. / 65400821598.),
-                c4 = F(-2691868925. / 45128329728.),
-                c5 = F(187940372067. / 1594534317056.),
-                c6 = F(-1776094331. / 19743644256.), c7 = F(11237099. / 235043384.);
-
-    F3 const uniform{F(rhs.field.x), F(rhs.field.y), F(rhs.field.z)};
-    F const coeffi = F(rhs.coeffi);
-    // Start position in FP32, for field-map lookups only
-    F3 const p0{F(beg_state.pos.x), F(beg_state.pos.y), F(beg_state.pos.z)};
-    // d(pos)/ds = p/|p|, d(mom)/ds = (q/|p|) p x B(pos), at the stage's
-    // position increment 'dp' from the start
-    auto eval = [&](F3 const& dp, F3 const& m, F3* kpos, F3* kmom) {
-        F3 const field
-            = rhs.map ? rzmap_field_f(*rhs.map, F3{p0.x + dp.x, p0.y + dp.y, p0.z + dp.z})
-                      : uniform;
-        F const inv = div(F(1), gbx::sqrt(m.x * m.x + m.y * m.y + m.z * m.z));
-        *kpos = {m.x * inv, m.y * inv, m.z * inv};
-        F const scale = coeffi * inv;
-        *kmom = {scale * (m.y * field.z - m.z * field.y),
-                 scale * (m.z * field.x - m.x * field.z),
-                 scale * (m.x * field.y - m.y * field.x)};
-    };
-    // Stage momentum m0 + h * sum_j a[j] k_mom[j]
-    auto stage = [](F3 const& m0, F h, F const* a, int n, F3 const* k) {
-        F3 r = m0;
-#pragma unroll
-        for (int j = 0; j < n; ++j)
-        {
-            r.x += h * a[j] * k[j].x;
-            r.y += h * a[j] * k[j].y;
-            r.z += h * a[j] * k[j].z;
-        }
-        return r;
-    };
-    F const A1[1] = {a11};
-    F const A2[2] = {a21, a22};
-    F const A3[3] = {a31, a32, a33};
-    F const A4[4] = {a41, a42, a43, a44};
-    F const A5[5] = {a51, a52, a53, a54, a55};
-
-    F const h = F(step);
-    F3 const m0{F(beg_state.mom.x), F(beg_state.mom.y), F(beg_state.mom.z)};
-    F3 const zero{0, 0, 0};
-    F3 kp[7], km[7];
-    // Stage position increments matter only for a field map
-    auto dpos_at = [&](F const* a, int n) {
-        return rhs.map ? stage(zero, h, a, n, kp) : zero;
-    };
-    eval(zero, m0, &kp[0], &km[0]);
-    eval(dpos_at(A1, 1), stage(m0, h, A1, 1, km), &kp[1], &km[1]);
-    eval(dpos_at(A2, 2), stage(m0, h, A2, 2, km), &kp[2], &km[2]);
-    eval(dpos_at(A3, 3), stage(m0, h, A3, 3, km), &kp[3], &km[3]);
-    eval(dpos_at(A4, 4), stage(m0, h, A4, 4, km), &kp[4], &km[4]);
-    eval(dpos_at(A5, 5), stage(m0, h, A5, 5, km), &kp[5], &km[5]);
-    // Fifth-order solution: FP32 increments added to the FP64 start
-    F const bf[7] = {F(b1), 0, F(b3), F(b4), F(b5), F(b6), 0};
-    F3 dpos{0, 0, 0}, m_end = m0;
-#pragma unroll
-    for (int i = 0; i < 6; ++i)
-    {
-        dpos.x += bf[i] * kp[i].x;
-        dpos.y += bf[i] * kp[i].y;
-        dpos.z += bf[i] * kp[i].z;
-        m_end.x += h * bf[i] * km[i].x;
-        m_end.y += h * bf[i] * km[i].y;
-        m_end.z += h * bf[i] * km[i].z;
-    }
-    F3 const end_inc{h * dpos.x, h * dpos.y, h * dpos.z};
-    eval(end_inc, m_end, &kp[6], &km[6]);
-
-    FieldStepperResult result;
-    result.end_state.pos = {beg_state.pos.x + double(end_inc.x),
-                            beg_state.pos.y + double(end_inc.y),
-                            beg_state.pos.z + double(end_inc.z)};
-    result.end_state.mom = {double(m_end.x), double(m_end.y), double(m_end.z)};
-
-    // Embedded error estimate: difference of the fifth- and fourth-order
-    // solutions, sum_i d_i k_i (times the step for the momentum)
-    F const df[7] = {F(d1), 0, F(d3), F(d4), F(d5), F(d6), F(d7)};
-    F3 epos{0, 0, 0}, emom{0, 0, 0};
-#pragma unroll
-    for (int i = 0; i < 7; ++i)
-    {
-        if (i == 1)
-            continue;
-        epos.x += df[i] * kp[i].x;
-        epos.y += df[i] * kp[i].y;
-        epos.z += df[i] * kp[i].z;
-        emom.x += df[i] * km[i].x;
-        emom.y += df[i] * km[i].y;
-        emom.z += df[i] * km[i].z;
-    }
-    result.err_pos_rate = epos;
-    result.err_mom = {h * emom.x, h * emom.y, h * emom.z};
-
-    // Shampine midpoint increment, and its distance from the chord
-    F const cf[7] = {c1, 0, c3, c4, c5, c6, c7};
-    F3 mpos{0, 0, 0};
-#pragma unroll
-    for (int i = 0; i < 7; ++i)
-    {
-        mpos.x += cf[i] * kp[i].x;
-        mpos.y += cf[i] * kp[i].y;
-        mpos.z += cf[i] * kp[i].z;
-    }
-    F const half = F(0.5) * h;
-    F3 const mid_inc{half * mpos.x, half * mpos.y, half * mpos.z};
-    F3 const cr{end_inc.y * mid_inc.z - end_inc.z * mid_inc.y,
-                end_inc.z * mid_inc.x - end_inc.x * mid_inc.z,
-                end_inc.x * mid_inc.y - end_inc.y * mid_inc.x};
-    result.dchord = gbx::sqrt(div(cr.x * cr.x + cr.y * cr.y + cr.z * cr.z,
-                                  end_inc.x * end_inc.x + end_inc.y * end_inc.y
-                                      + end_inc.z * end_inc.z));
-    return result;
-}
-
-//! Dormand-Prince step of this build's precision
+//! Dormand-Prince step with the problem's field source
 GBX_FORCEINLINE FieldStepperResult dormand_prince_step(UniformFieldEquation const& rhs,
                                                        double step,
                                                        OdeState const& beg_state)
 {
-    if constexpr (sizeof(real_type) == sizeof(double))
-    {
-        if (rhs.map)
-            return dormand_prince_step_fp64(FixedFieldEquation<true>{rhs}, step, beg_state);
-        return dormand_prince_step_fp64(FixedFieldEquation<false>{rhs}, step, beg_state);
-    }
-    else
-    {
-        return dormand_prince_step_mixed(rhs, step, beg_state);
-    }
+    if (rhs.map)
+        return dormand_prince_step_fp64(FixedFieldEquation<true>{rhs}, step, beg_state);
+    return dormand_prince_step_fp64(FixedFieldEquation<false>{rhs}, step, beg_state);
 }
 
 //---------------------------------------------------------------------------//
 // Field driver
 //---------------------------------------------------------------------------//
-struct DriverResult
-{
-    OdeState state;
-    double step;
-};
-
 class FieldDriver
 {
   public:
@@ -499,35 +277,14 @@ class FieldDriver
                                        double step,
                                        Real3 const& mom) const
     {
-        if constexpr (sizeof(real_type) == sizeof(double))
-        {
-            return div(rel_err_sq(result.err_state, step, mom),
-                       ipow<2>(opt_.epsilon_rel_max));
-        }
-        else
-        {
-            // FP64 norms of the FP32 error estimate; the position error
-            // comes as a rate, so no division by the step is needed
-            Real3 const ep{double(result.err_pos_rate.x),
-                           double(result.err_pos_rate.y),
-                           double(result.err_pos_rate.z)};
-            Real3 const em{double(result.err_mom.x),
-                           double(result.err_mom.y),
-                           double(result.err_mom.z)};
-            double const errpos2 = dot_product(ep, ep);
-            double const errvel2 = div(dot_product(em, em), dot_product(mom, mom));
-            return div(max_of(errpos2, errvel2), ipow<2>(opt_.epsilon_rel_max));
-        }
+        return div(rel_err_sq(result.err_state, step, mom), ipow<2>(opt_.epsilon_rel_max));
     }
 
     //! Distance of the stepper's midpoint from the chord
     GBX_FORCEINLINE double chord_distance(FieldStepperResult const& result,
                                           OdeState const& state) const
     {
-        if constexpr (sizeof(real_type) == sizeof(double))
-            return distance_chord(state.pos, result.mid_state.pos, result.end_state.pos);
-        else
-            return double(result.dchord);
+        return distance_chord(state.pos, result.mid_state.pos, result.end_state.pos);
     }
 
     static GBX_FORCEINLINE double distance_chord(Real3 const& beg_pos,
@@ -543,17 +300,7 @@ class FieldDriver
     GBX_FORCEINLINE double new_step_scale(double err_sq) const
     {
         double const power = 0.5 * (err_sq > 1 ? opt_.pshrink : opt_.pgrow);
-        if constexpr (sizeof(real_type) == sizeof(double))
-        {
-            return opt_.safety * fastpow(err_sq, power);
-        }
-        else
-        {
-            // Heuristic step-size factor in FP32 (the acceptance test that
-            // uses err_sq stays FP64); clamp the argument to FP32 range
-            float const e = float(min_of(max_of(err_sq, 1e-30), 1e30));
-            return opt_.safety * double(libm::exp(float(power) * libm::log(e)));
-        }
+        return opt_.safety * fastpow(err_sq, power);
     }
 
     GBX_FUNCTION ChordSearch find_next_chord(double step, OdeState const& state) const
@@ -678,7 +425,8 @@ inline unsigned long long safe_ball_mismatches = 0;
 //! split into its set-up, one substep of its loop and its completion so that
 //! a kernel can interleave the substeps of different tracks. Running
 //! init(), then substep() until done(), then finish() is the reference's
-//! sequence of operations.
+//! sequence of operations. RoundX is the mixed-precision driver's.
+template<bool RoundX = true>
 class FieldPropagation
 {
   public:
@@ -720,7 +468,7 @@ class FieldPropagation
     }
 
     //! One iteration of the substep loop
-    GBX_FUNCTION void substep(GeoTrackView& geo)
+    GBX_FORCEINLINE void substep(GeoTrackView& geo)
     {
         double const delta_intersection = driver_.delta_intersection();
         double const minimum_substep = driver_.minimum_step();
@@ -758,7 +506,7 @@ class FieldPropagation
         // queries the ball would have answered and any it would have got
         // wrong
         bool const ball = this->inside_safe_ball(geo, max_dist);
-        Propagation linear_step = geo.find_next_step(max_dist);
+        Propagation linear_step = geo.find_next_step<false>(max_dist);
         if (ball)
         {
             ++safe_ball_uses;
@@ -768,7 +516,7 @@ class FieldPropagation
 #else
         Propagation linear_step = this->inside_safe_ball(geo, max_dist)
                                       ? geo.no_crossing(max_dist)
-                                      : geo.find_next_step(max_dist);
+                                      : geo.find_next_step<false>(max_dist);
 #endif
         if (!linear_step.boundary)
         {
@@ -817,7 +565,7 @@ class FieldPropagation
     }
 
     //! Complete the propagation after the loop
-    GBX_FUNCTION Propagation finish(GeoTrackView& geo)
+    GBX_FORCEINLINE Propagation finish(GeoTrackView& geo)
     {
         double const bump_distance = driver_.delta_intersection() * double(0.1);
         if (remaining_substeps_ == 0 && result_.distance < step_)
@@ -877,7 +625,7 @@ class FieldPropagation
     //! least the safety distance (|x - v|, |r - R|) from the centre. A
     //! safety the multiple-scattering step limit measured at the start
     //! gives the ball from the first substep on.
-    GBX_FUNCTION bool inside_safe_ball(GeoTrackView& geo, double max_dist)
+    GBX_FORCEINLINE bool inside_safe_ball(GeoTrackView& geo, double max_dist)
     {
         if (safe_radius_ < 0 || !geo.is_clear_of_boundary())
             return false;
@@ -906,7 +654,8 @@ class FieldPropagation
   public:
 
   private:
-    FieldDriver driver_;
+    std::conditional_t<sizeof(real_type) == sizeof(double), FieldDriver, MixedFieldDriver<RoundX>>
+        driver_;
     OdeState state_;
     Propagation result_;
     //! Ball free of surfaces: its center and radius (0: not yet measured,
@@ -926,7 +675,7 @@ GBX_FUNCTION Propagation propagate_in_field(FieldOptions const& opt,
                                             GeoTrackView& geo,
                                             double step)
 {
-    FieldPropagation fp(opt, rhs);
+    FieldPropagation<> fp(opt, rhs);
     fp.init(geo, momentum, step);
     do
     {

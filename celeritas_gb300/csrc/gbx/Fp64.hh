@@ -153,13 +153,11 @@ GBX_FORCEINLINE std::uint64_t sqrt_significand(std::uint64_t m, std::uint32_t y)
     return (s + 1) >> 1;
 }
 
-}  // namespace fp64
 
-//! a / b, correctly rounded
-GBX_NOINLINE double div(double a, double b)
+//! a / b, correctly rounded, inlined: for a loop that one track waits for
+GBX_FORCEINLINE double div_inline(double a, double b)
 {
 #if defined(__CUDA_ARCH__)
-    using namespace fp64;
     std::uint64_t const ua = __double_as_longlong(a);
     std::uint64_t const ub = __double_as_longlong(b);
     auto const ah = static_cast<std::uint32_t>(ua >> 32);
@@ -184,11 +182,10 @@ GBX_NOINLINE double div(double a, double b)
 #endif
 }
 
-//! Square root, correctly rounded
-GBX_NOINLINE double sqrt(double a)
+//! Square root, correctly rounded, inlined
+GBX_FORCEINLINE double sqrt_inline(double a)
 {
 #if defined(__CUDA_ARCH__)
-    using namespace fp64;
     std::uint64_t const ua = __double_as_longlong(a);
     auto const ah = static_cast<std::uint32_t>(ua >> 32);
     // Positive and normal
@@ -210,6 +207,49 @@ GBX_NOINLINE double sqrt(double a)
 #endif
 }
 
+//! The FP32 value nearest to a positive double (ties to even)
+GBX_FORCEINLINE float narrow(double a)
+{
+#if defined(__CUDA_ARCH__)
+    std::uint64_t const u = __double_as_longlong(a);
+    auto const hi = static_cast<std::uint32_t>(u >> 32);
+    // In the range of FP32's normal numbers: rebias, round to 24 bits
+    if (hi - 0x38100000u < 0x0fe00000u)
+    {
+        std::uint64_t const t = u - (std::uint64_t(0x38000000u) << 32) + 0x0fffffffu
+                                + ((u >> 29) & 1u);
+        return __uint_as_float(static_cast<std::uint32_t>(t >> 29));
+    }
+#endif
+    return static_cast<float>(a);
+}
+
+//! The double equal to a positive FP32 number
+GBX_FORCEINLINE double widen(float a)
+{
+#if defined(__CUDA_ARCH__)
+    std::uint32_t const u = __float_as_uint(a);
+    // Normal numbers: rebias
+    if (u - 0x00800000u < 0x7f000000u)
+    {
+        return __hiloint2double(static_cast<int>((u >> 3) + 0x38000000u),
+                                static_cast<int>(u << 29));
+    }
+#endif
+    return a;
+}
+}  // namespace fp64
+
+//! a / b, correctly rounded
+GBX_NOINLINE double div(double a, double b)
+{
+    return fp64::div_inline(a, b);
+}
+//! Square root, correctly rounded
+GBX_NOINLINE double sqrt(double a)
+{
+    return fp64::sqrt_inline(a);
+}
 GBX_FORCEINLINE float div(float a, float b)
 {
     return a / b;

@@ -150,6 +150,9 @@ class GeoTrackView
     }
 
     //// NAVIGATION ////
+    //! Contract: in the mixed build, 1 - (dir . z)^2 of the background search may
+    //! be one fma (FieldPropagation's query has always rounded the square)
+    template<bool Contract = true>
     GBX_FUNCTION Propagation find_next_step(double max_step);
     GBX_FUNCTION void move_to_boundary();
     GBX_FUNCTION void move_internal(double dist);
@@ -215,6 +218,7 @@ class GeoTrackView
     //! whose nearest point is farther than max_dist are skipped without
     //! solving: every distance along the ray is at least that far, so the
     //! caller's "d <= max_dist" test would reject them anyway.
+    template<bool Contract = true>
     GBX_FUNCTION void intersect(size_type surf,
                                 Real3 const& pos,
                                 Real3 const& dir,
@@ -262,7 +266,11 @@ class GeoTrackView
                 return;
         }
         // 1 - (dir . z)^2; no intersection when traveling along the axis
-        double const a = 1 - ipow<2>(dir.z);
+        double a;
+        if constexpr (Contract)
+            a = 1 - ipow<2>(dir.z);
+        else
+            a = sub_rounded(1, mul_rounded(dir.z, dir.z));
         constexpr double sqrt_quadratic = 1e-5;
         if (a < ipow<2>(sqrt_quadratic))
             return;
@@ -318,6 +326,7 @@ class GeoTrackView
                                         double bump,
                                         double max_step,
                                         Crossing* hit) const;
+    template<bool Contract>
     GBX_FUNCTION void background_crossing(Real3 const& pos,
                                           Real3 const& dir,
                                           size_type cur_surf,
@@ -516,6 +525,7 @@ GBX_FUNCTION size_type GeoTrackView::find_volume_at(Real3 const& pos,
 }
 
 //---------------------------------------------------------------------------//
+template<bool Contract>
 GBX_FUNCTION Propagation GeoTrackView::find_next_step(double max_step)
 {
     Propagation result{max_step, false, false};
@@ -572,7 +582,7 @@ GBX_FUNCTION Propagation GeoTrackView::find_next_step(double max_step)
     else
     {
         Crossing hit{invalid_id, max_step, 0};
-        this->background_crossing(pos, dir, cur_surf, max_step, &hit);
+        this->background_crossing<Contract>(pos, dir, cur_surf, max_step, &hit);
         hit_surf = hit.surf;
         hit_dist = hit.dist;
         hit_sense = hit.sense;
@@ -673,6 +683,7 @@ GBX_FUNCTION void GeoTrackView::consider_crossing(size_type surf,
 //! R| stops a cylinder walk only where every root is beyond the limit, with
 //! the same margin as the per-surface reachability test. The result is
 //! therefore the crossing a solve of every surface would give.
+template<bool Contract>
 GBX_FUNCTION void GeoTrackView::background_crossing(Real3 const& pos,
                                                     Real3 const& dir,
                                                     size_type cur_surf,
@@ -690,7 +701,7 @@ GBX_FUNCTION void GeoTrackView::background_crossing(Real3 const& pos,
     for (size_type surf = 0; surf < p_.num_surfaces; ++surf)
     {
         double dd[2];
-        this->intersect(surf, pos, dir, surf == cur_surf, dd, max_step);
+        this->intersect<Contract>(surf, pos, dir, surf == cur_surf, dd, max_step);
         for (int k = 0; k < 2; ++k)
             this->consider_crossing(surf, dd[k], pos, dir, bump, max_step, hit);
     }
@@ -704,7 +715,7 @@ GBX_FUNCTION void GeoTrackView::background_crossing(Real3 const& pos,
     if (cur_surf != invalid_id)
     {
         double dd[2];
-        this->intersect(cur_surf, pos, dir, true, dd);
+        this->intersect<Contract>(cur_surf, pos, dir, true, dd);
         for (int k = 0; k < 2; ++k)
             this->consider_crossing(cur_surf, dd[k], pos, dir, bump, max_step, hit);
     }
@@ -741,7 +752,7 @@ GBX_FUNCTION void GeoTrackView::background_crossing(Real3 const& pos,
             if (rf - key[i] - radial_margin(key[i], limit_f) > limit_f)
                 break;
             double dd[2];
-            this->intersect(surf, pos, dir, false, dd);
+            this->intersect<Contract>(surf, pos, dir, false, dd);
             if (dd[0] < INFINITY)
             {
                 if (dd[0] > limit)
@@ -773,7 +784,7 @@ GBX_FUNCTION void GeoTrackView::background_crossing(Real3 const& pos,
             if (key[i] - rf - radial_margin(key[i], limit_f) > limit_f)
                 break;
             double dd[2];
-            this->intersect(surf, pos, dir, false, dd);
+            this->intersect<Contract>(surf, pos, dir, false, dd);
             double const far = (dd[1] < INFINITY) ? dd[1] : dd[0];
             if (!(far < INFINITY))
             {

@@ -91,6 +91,24 @@ GBX_FORCEINLINE float gbx_fma(float a, float b, float c)
     return ::fmaf(a, b, c);
 }
 
+//! Product and difference rounded one by one, never contracted
+GBX_FORCEINLINE double mul_rounded(double a, double b)
+{
+#if defined(__CUDA_ARCH__)
+    return __dmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+GBX_FORCEINLINE double sub_rounded(double a, double b)
+{
+#if defined(__CUDA_ARCH__)
+    return __dsub_rn(a, b);
+#else
+    return a - b;
+#endif
+}
+
 //---------------------------------------------------------------------------//
 // Three-vector
 //---------------------------------------------------------------------------//

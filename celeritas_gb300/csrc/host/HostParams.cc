@@ -506,6 +506,7 @@ void Builder::build_physics()
     if (!opts_.field_options.valid())
         throw std::runtime_error("invalid field driver options");
     s.field_options = opts_.field_options;
+    s.field_options.derive();
     // PhysicsParamsOptions defaults and imported EM parameters
     s.min_range = 1 * constants::millimeter;
     s.max_step_over_range = 0.2;
@@ -828,6 +829,9 @@ void Builder::read_rzmap(std::string const& path)
         g.back = hi;
         g.delta = (hi - lo) / (n - 1);
         g.size = n;
+        g.front_f = static_cast<float>(g.front);
+        g.back_f = static_cast<float>(g.back);
+        g.delta_f = static_cast<float>(g.delta);
         return g;
     };
     hp_.rzmap_desc.z = grid(min_z, max_z, nz);
