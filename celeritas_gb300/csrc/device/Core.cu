@@ -88,6 +88,8 @@ class KernelAction : public CoreStepActionInterface, public ConcreteAction
             launch_(params, state, this->action_id());
     }
 
+    Launch launch() const { return launch_; }
+
   private:
     StepActionOrder order_;
     Launch launch_;
@@ -494,6 +496,7 @@ CoreState::CoreState(CoreParams const& params,
     std::size_t o_tslots = arr(4);
     std::size_t o_aoff = L.reserve(4 * 2 * std::size_t(num_bins + 1));
     std::size_t o_shist = L.reserve(4 * std::size_t(num_bins) * sort_blocks);
+    std::size_t o_stot = L.reserve(4 * std::size_t(num_bins));
     std::size_t o_work = L.reserve(sizeof(size_type));
     std::size_t o_log = L.reserve(sizeof(StepRecord) * log_cap);
     std::size_t o_stepidx = L.reserve(sizeof(size_type));
@@ -651,6 +654,7 @@ CoreState::CoreState(CoreParams const& params,
     ctx_.scratch.count = static_cast<size_type*>(at(o_scnt));
     ctx_.scratch.num_blocks = nblocks;
     ctx_.sort.block_hist = static_cast<size_type*>(at(o_shist));
+    ctx_.sort.bin_totals = static_cast<size_type*>(at(o_stot));
     ctx_.sort.num_bins = num_bins;
     ctx_.sort.num_blocks = sort_blocks;
     ctx_.sort.num_actions = num_actions;
@@ -1190,8 +1194,22 @@ void ActionSequence::step(CoreParams const& params, CoreState& state) const
 {
     if (!timing_)
     {
+        // The model actions follow one another and a track interacts by one of
+        // them, so one launch over all their tracks does the same as one per
+        // model, without the others' launches and waits for their last warps
+        bool models_done = false;
         for (auto const* a : actions_)
+        {
+            auto const* kernel = dynamic_cast<KernelAction const*>(a);
+            if (kernel && kernel->launch() == step_model)
+            {
+                if (!models_done)
+                    launch_interact(state.context(), invalid_id, state.stream());
+                models_done = true;
+                continue;
+            }
             a->step(params, state);
+        }
         return;
     }
     // Events bracket each action on the state's stream; accumulate the

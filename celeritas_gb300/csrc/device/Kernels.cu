@@ -87,6 +87,71 @@ __device__ __forceinline__ size_type block_exclusive_scan(size_type value,
     return result;
 }
 
+//! Exclusive scan of one value per thread of a 1024-thread block: two warp
+//! shuffle scans and three barriers
+struct WideScanStorage
+{
+    size_type warp_sums[32];
+    size_type total;
+};
+
+__device__ __forceinline__ size_type wide_exclusive_scan(size_type value, WideScanStorage& tmp)
+{
+    unsigned int const lane = threadIdx.x & 31u;
+    unsigned int const warp = threadIdx.x >> 5;
+    auto warp_inclusive = [lane](size_type v) {
+#pragma unroll
+        for (unsigned int offset = 1; offset < 32; offset <<= 1)
+        {
+            size_type const n = __shfl_up_sync(0xffffffffu, v, offset);
+            if (lane >= offset)
+                v += n;
+        }
+        return v;
+    };
+    size_type const incl = warp_inclusive(value);
+    if (lane == 31)
+        tmp.warp_sums[warp] = incl;
+    __syncthreads();
+    if (warp == 0)
+    {
+        size_type const w = tmp.warp_sums[lane];
+        size_type const wincl = warp_inclusive(w);
+        tmp.warp_sums[lane] = wincl - w;
+        if (lane == 31)
+            tmp.total = wincl;
+    }
+    __syncthreads();
+    size_type const result = tmp.warp_sums[warp] + incl - value;
+    __syncthreads();
+    return result;
+}
+
+//! Exclusive scan in place of n values by one 1024-thread block, starting from
+//! 'first'; returns the sum of all. Each thread takes a run of consecutive
+//! values and the runs' sums are scanned once, where a pass of 1024 values at a
+//! time would need its barriers for each.
+__device__ __forceinline__ size_type scan_in_place(size_type* values,
+                                                   size_type n,
+                                                   size_type first,
+                                                   WideScanStorage& tmp)
+{
+    size_type const per = (n + 1023) / 1024;
+    size_type const begin = min_of(n, threadIdx.x * per);
+    size_type const end = min_of(n, begin + per);
+    size_type sum = 0;
+    for (size_type i = begin; i < end; ++i)
+        sum += values[i];
+    size_type run = first + wide_exclusive_scan(sum, tmp);
+    for (size_type i = begin; i < end; ++i)
+    {
+        size_type const v = values[i];
+        values[i] = run;
+        run += v;
+    }
+    return first + tmp.total;
+}
+
 //---------------------------------------------------------------------------//
 // Primaries and track initialization
 //---------------------------------------------------------------------------//
@@ -222,33 +287,10 @@ __global__ __launch_bounds__(block_size) void charge_partition_count_kernel(
 __global__ __launch_bounds__(1024) void charge_partition_scan_kernel(ScanScratch scr)
 {
     // Exclusive scan of the per-block neutral counts by one block
-    __shared__ size_type sh[1024];
-    __shared__ size_type carry;
+    __shared__ WideScanStorage tmp;
+    size_type const total = scan_in_place(scr.block_vacant, scr.num_blocks, 0, tmp);
     if (threadIdx.x == 0)
-        carry = 0;
-    __syncthreads();
-    for (size_type base = 0; base < scr.num_blocks; base += 1024)
-    {
-        size_type const i = base + threadIdx.x;
-        size_type const v = i < scr.num_blocks ? scr.block_vacant[i] : 0;
-        sh[threadIdx.x] = v;
-        __syncthreads();
-        for (int off = 1; off < 1024; off <<= 1)
-        {
-            size_type const a = threadIdx.x >= off ? sh[threadIdx.x - off] : 0;
-            __syncthreads();
-            sh[threadIdx.x] += a;
-            __syncthreads();
-        }
-        if (i < scr.num_blocks)
-            scr.block_vacant[i] = carry + sh[threadIdx.x] - v;
-        __syncthreads();
-        if (threadIdx.x == 1023)
-            carry += sh[1023];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        scr.count[0] = carry;
+        scr.count[0] = total;
 }
 
 __global__ __launch_bounds__(block_size) void charge_partition_scatter_kernel(
@@ -415,38 +457,15 @@ __global__ __launch_bounds__(1024) void hits_scan_kernel(StateData s,
                                                          size_type num_blocks,
                                                          size_type capacity)
 {
-    __shared__ size_type sh[1024];
-    __shared__ size_type carry;
+    __shared__ WideScanStorage tmp;
     Counters& c = *s.counters;
-    if (threadIdx.x == 0)
-        carry = c.num_hits;
-    __syncthreads();
-    for (size_type base = 0; base < num_blocks; base += 1024)
-    {
-        size_type const i = base + threadIdx.x;
-        size_type const v = i < num_blocks ? block_hits[i] : 0;
-        sh[threadIdx.x] = v;
-        __syncthreads();
-        for (int off = 1; off < 1024; off <<= 1)
-        {
-            size_type const a = threadIdx.x >= off ? sh[threadIdx.x - off] : 0;
-            __syncthreads();
-            sh[threadIdx.x] += a;
-            __syncthreads();
-        }
-        if (i < num_blocks)
-            block_hits[i] = carry + sh[threadIdx.x] - v;
-        __syncthreads();
-        if (threadIdx.x == 1023)
-            carry += sh[1023];
-        __syncthreads();
-    }
+    size_type const total = scan_in_place(block_hits, num_blocks, c.num_hits, tmp);
     if (threadIdx.x == 0)
     {
-        if (carry > capacity)
+        if (total > capacity)
             c.error_flags |= error_hit_overflow;
         else if (!(c.error_flags & error_hit_overflow))
-            c.num_hits = carry;
+            c.num_hits = total;
     }
 }
 
@@ -536,46 +555,10 @@ __global__ __launch_bounds__(1024) void scan_blocks_kernel(StateData s,
                                                            size_type* step_index)
 {
     // Exclusive scan of the per-block totals by one block of 1024 threads
-    __shared__ size_type sh_vac[1024];
-    __shared__ size_type sh_cnt[1024];
-    __shared__ size_type carry_vac, carry_cnt;
-    if (threadIdx.x == 0)
-    {
-        carry_vac = 0;
-        carry_cnt = 0;
-    }
-    __syncthreads();
-    for (size_type base = 0; base < scr.num_blocks; base += 1024)
-    {
-        size_type i = base + threadIdx.x;
-        size_type v = i < scr.num_blocks ? scr.block_vacant[i] : 0;
-        size_type c = i < scr.num_blocks ? scr.block_count[i] : 0;
-        sh_vac[threadIdx.x] = v;
-        sh_cnt[threadIdx.x] = c;
-        __syncthreads();
-        // Hillis-Steele inclusive scan
-        for (int off = 1; off < 1024; off <<= 1)
-        {
-            size_type av = threadIdx.x >= off ? sh_vac[threadIdx.x - off] : 0;
-            size_type ac = threadIdx.x >= off ? sh_cnt[threadIdx.x - off] : 0;
-            __syncthreads();
-            sh_vac[threadIdx.x] += av;
-            sh_cnt[threadIdx.x] += ac;
-            __syncthreads();
-        }
-        if (i < scr.num_blocks)
-        {
-            scr.block_vacant[i] = carry_vac + sh_vac[threadIdx.x] - v;
-            scr.block_count[i] = carry_cnt + sh_cnt[threadIdx.x] - c;
-        }
-        __syncthreads();
-        if (threadIdx.x == 1023)
-        {
-            carry_vac += sh_vac[1023];
-            carry_cnt += sh_cnt[1023];
-        }
-        __syncthreads();
-    }
+    __shared__ WideScanStorage tmp_vac;
+    __shared__ WideScanStorage tmp_cnt;
+    size_type const carry_vac = scan_in_place(scr.block_vacant, scr.num_blocks, 0, tmp_vac);
+    size_type const carry_cnt = scan_in_place(scr.block_count, scr.num_blocks, 0, tmp_cnt);
     if (threadIdx.x == 0)
     {
         Counters& c = *s.counters;
@@ -657,8 +640,8 @@ __global__ void kill_active_kernel(ParamsData p, StateData s)
 //---------------------------------------------------------------------------//
 // Action sort (SortTracksAction): stable counting sort of the track slots by
 // action ID in three kernels. Blocks of sort_block_size slots count their
-// keys with warp-aggregated shared-memory atomics (match_any + popc); one
-// block scans the bin-major [bin][block] counts; the scatter ranks each slot
+// keys with warp-aggregated shared-memory atomics (match_any + popc); one block
+// per bin scans its row of the [bin][block] counts; the scatter ranks each slot
 // among equal keys of its warp (match_any) and of the preceding warps, so
 // slots of one action stay in increasing order.
 //---------------------------------------------------------------------------//
@@ -712,64 +695,53 @@ __global__ __launch_bounds__(sort_block_size) void sort_count_kernel(
         srt.block_hist[i * srt.num_blocks + blockIdx.x] = hist[i];
 }
 
-__global__ __launch_bounds__(1024) void sort_scan_kernel(StateData s,
-                                                         SortScratch srt,
-                                                         size_type* offsets)
+//! One block per bin: exclusive scan of the bin's counts over the slot blocks
+//! and the bin's total; the scatter adds the totals of the bins before. With a
+//! single block over all bins, whose threads each read a run of their own, a sort
+//! of 2^20 slots took 66 us (three launches, event times), with one bin per
+//! block 22.
+__global__ __launch_bounds__(1024) void sort_scan_kernel(SortScratch srt)
 {
-    __shared__ size_type warp_sums[32];
-    size_type const total = srt.num_bins * srt.num_blocks;
-    size_type const per = (total + 1023) / 1024;
-    size_type const begin = min_of(total, threadIdx.x * per);
-    size_type const end = min_of(total, begin + per);
-    size_type sum = 0;
-    for (size_type i = begin; i < end; ++i)
-        sum += srt.block_hist[i];
-    // Block-wide exclusive scan of the per-thread sums
-    unsigned int const lane = threadIdx.x & 31u;
-    unsigned int const warp = threadIdx.x >> 5;
-    size_type incl = sum;
-    for (unsigned int off = 1; off < 32; off <<= 1)
-    {
-        size_type v = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off)
-            incl += v;
-    }
-    if (lane == 31)
-        warp_sums[warp] = incl;
-    __syncthreads();
-    if (warp == 0)
-    {
-        size_type const w = warp_sums[lane];
-        size_type wi = w;
-        for (unsigned int off = 1; off < 32; off <<= 1)
-        {
-            size_type v = __shfl_up_sync(0xffffffffu, wi, off);
-            if (lane >= off)
-                wi += v;
-        }
-        warp_sums[lane] = wi - w;
-    }
-    __syncthreads();
-    size_type run = warp_sums[warp] + incl - sum;
-    for (size_type i = begin; i < end; ++i)
-    {
-        size_type const c = srt.block_hist[i];
-        srt.block_hist[i] = run;
-        run += c;
-    }
-    __syncthreads();
-    for (size_type b = threadIdx.x; b < srt.num_bins; b += blockDim.x)
-        offsets[b] = srt.block_hist[b * srt.num_blocks];
+    __shared__ WideScanStorage tmp;
+    size_type const total = scan_in_place(
+        srt.block_hist + std::size_t(blockIdx.x) * srt.num_blocks, srt.num_blocks, 0, tmp);
     if (threadIdx.x == 0)
-        offsets[srt.num_bins] = s.size;
+        srt.bin_totals[blockIdx.x] = total;
 }
 
 __global__ __launch_bounds__(sort_block_size) void sort_scatter_kernel(
-    StateData s, SortScratch srt, SortKey key)
+    StateData s, SortScratch srt, SortKey key, size_type* offsets)
 {
     constexpr unsigned int num_warps = sort_block_size / 32;
-    extern __shared__ size_type warp_hist[];  // [num_warps][num_bins]
+    extern __shared__ size_type warp_hist[];  // [num_warps][num_bins], [num_bins]
     size_type const nb = srt.num_bins;
+    size_type* const bin_base = warp_hist + num_warps * nb;
+    if (threadIdx.x < 32)
+    {
+        // First position of each bin: exclusive scan of the totals
+        size_type before = 0;
+        for (size_type first = 0; first < nb; first += 32)
+        {
+            size_type const b = first + threadIdx.x;
+            size_type const v = b < nb ? srt.bin_totals[b] : 0;
+            size_type incl = v;
+            for (unsigned int off = 1; off < 32; off <<= 1)
+            {
+                size_type const n = __shfl_up_sync(0xffffffffu, incl, off);
+                if (threadIdx.x >= off)
+                    incl += n;
+            }
+            if (b < nb)
+            {
+                bin_base[b] = before + incl - v;
+                if (blockIdx.x == 0)
+                    offsets[b] = before + incl - v;
+            }
+            before += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            offsets[nb] = s.size;
+    }
     for (size_type i = threadIdx.x; i < num_warps * nb; i += blockDim.x)
         warp_hist[i] = 0;
     __syncthreads();
@@ -796,7 +768,7 @@ __global__ __launch_bounds__(sort_block_size) void sort_scatter_kernel(
     __syncthreads();
     if (valid)
     {
-        size_type const pos = srt.block_hist[k * srt.num_blocks + blockIdx.x]
+        size_type const pos = bin_base[k] + srt.block_hist[k * srt.num_blocks + blockIdx.x]
                               + warp_hist[warp * nb + k] + __popc(lower);
         s.track_slots[pos] = slot;
     }
@@ -1133,7 +1105,10 @@ void launch_interact(LaunchContext const& ctx, size_type action, cudaStream_t st
     size_type first = action, end = action + 1;
     if (action == invalid_id)
     {
-        // All models at once: they are mutually exclusive per slot
+        // All models at once: they are mutually exclusive per slot. A step's
+        // seven launches become one: 100 electrons of 1 GeV in FP64 49 -> 37
+        // ms, 3000 c2 electrons in the mixed build (with the sort's scan)
+        // 207 -> 166 ms.
         first = p.model_to_action;
         end = p.model_to_action + p.num_models;
     }
@@ -1268,11 +1243,11 @@ void launch_sort_tracks(LaunchContext const& ctx, SortKey key, cudaStream_t stre
                         sort_block_size,
                         srt.num_bins * sizeof(size_type),
                         stream>>>(ctx.state, srt, key);
-    sort_scan_kernel<<<1, 1024, 0, stream>>>(ctx.state, srt, sort_offsets(ctx, key));
+    sort_scan_kernel<<<srt.num_bins, 1024, 0, stream>>>(srt);
     sort_scatter_kernel<<<srt.num_blocks,
                           sort_block_size,
-                          (sort_block_size / 32) * srt.num_bins * sizeof(size_type),
-                          stream>>>(ctx.state, srt, key);
+                          (sort_block_size / 32 + 1) * srt.num_bins * sizeof(size_type),
+                          stream>>>(ctx.state, srt, key, sort_offsets(ctx, key));
 }
 
 //---------------------------------------------------------------------------//

@@ -31,6 +31,7 @@ struct ScanScratch
 struct SortScratch
 {
     size_type* block_hist;  //!< [num_bins * num_blocks]
+    size_type* bin_totals;  //!< [num_bins]
     //! num_actions + num_materials + 1 (last: invalid action)
     size_type num_bins;
     size_type num_blocks;
