@@ -484,8 +484,8 @@ CoreState::CoreState(CoreParams const& params,
     std::size_t o_counters = L.reserve(sizeof(Counters));
     std::size_t o_bvac = L.reserve(4 * std::size_t(nblocks));
     std::size_t o_bcnt = L.reserve(4 * std::size_t(nblocks));
-    std::size_t o_svac = arr(1);
-    std::size_t o_scnt = arr(4);
+    std::size_t o_sflags = arr(1);
+    std::size_t o_ticket = L.reserve(sizeof(size_type));
     // Action sort: thread -> slot indirection, bin offsets, block counts
     size_type const num_actions = params.host().scalars.num_actions;
     size_type const num_materials = max_of<size_type>(1, params.host().scalars.num_materials);
@@ -650,8 +650,8 @@ CoreState::CoreState(CoreParams const& params,
     ctx_.state = s;
     ctx_.scratch.block_vacant = static_cast<size_type*>(at(o_bvac));
     ctx_.scratch.block_count = static_cast<size_type*>(at(o_bcnt));
-    ctx_.scratch.vacant = static_cast<std::uint8_t*>(at(o_svac));
-    ctx_.scratch.count = static_cast<size_type*>(at(o_scnt));
+    ctx_.scratch.flags = static_cast<std::uint8_t*>(at(o_sflags));
+    ctx_.scratch.ticket = static_cast<size_type*>(at(o_ticket));
     ctx_.scratch.num_blocks = nblocks;
     ctx_.sort.block_hist = static_cast<size_type*>(at(o_shist));
     ctx_.sort.bin_totals = static_cast<size_type*>(at(o_stot));
@@ -679,9 +679,9 @@ CoreState::CoreState(CoreParams const& params,
     ctx_.persistent_blocks = sizeof(real_type) < sizeof(double)
                                  ? persistent_along_blocks(ctx_.along_block_size)
                                  : 0;
-    ctx_.log = static_cast<StepRecord*>(at(o_log));
-    ctx_.log_capacity = log_cap;
-    ctx_.step_index = static_cast<size_type*>(at(o_stepidx));
+    ctx_.log.records = static_cast<StepRecord*>(at(o_log));
+    ctx_.log.capacity = log_cap;
+    ctx_.log.step_index = static_cast<size_type*>(at(o_stepidx));
 
     pinned_capacity_ = prim_cap;
     GBX_CUDA(cudaMallocHost(&pinned_primaries_,
@@ -1091,23 +1091,23 @@ size_type CoreState::step_index() const
 {
     size_type idx;
     GBX_CUDA(cudaMemcpyAsync(
-        &idx, ctx_.step_index, sizeof(idx), cudaMemcpyDeviceToHost, stream_));
+        &idx, ctx_.log.step_index, sizeof(idx), cudaMemcpyDeviceToHost, stream_));
     GBX_CUDA(cudaStreamSynchronize(stream_));
     return idx;
 }
 
 std::vector<StepRecord> CoreState::step_log(size_type first, size_type n) const
 {
-    std::vector<StepRecord> all(ctx_.log_capacity);
+    std::vector<StepRecord> all(ctx_.log.capacity);
     GBX_CUDA(cudaMemcpyAsync(all.data(),
-                             ctx_.log,
+                             ctx_.log.records,
                              sizeof(StepRecord) * all.size(),
                              cudaMemcpyDeviceToHost,
                              stream_));
     GBX_CUDA(cudaStreamSynchronize(stream_));
     std::vector<StepRecord> result(n);
     for (size_type i = 0; i < n; ++i)
-        result[i] = all[(first + i) % ctx_.log_capacity];
+        result[i] = all[(first + i) % ctx_.log.capacity];
     return result;
 }
 
@@ -1208,6 +1208,14 @@ void ActionSequence::step(CoreParams const& params, CoreState& state) const
                 models_done = true;
                 continue;
             }
+            // Boundary and cut follow one another too
+            if (kernel && kernel->launch() == step_boundary)
+            {
+                launch_boundary_cut(state.context(), state.stream());
+                continue;
+            }
+            if (kernel && kernel->launch() == step_cut)
+                continue;
             a->step(params, state);
         }
         return;

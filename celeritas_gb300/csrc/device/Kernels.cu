@@ -9,8 +9,7 @@
 // step, src/celeritas/track/detail/TrackInitAlgorithms.cu:34-78).
 //
 // End-of-step bookkeeping (src/celeritas/track/ExtendFromSecondariesAction.cc)
-// is three kernels: per-slot vacancy flags and secondary counts with
-// per-block totals (warp ballot/popc and shuffle scans), one block scanning
+// is three kernels: per-slot flags with per-block totals, one block scanning
 // the block totals and updating the counters, and a scatter that writes the
 // stably compacted vacancy list and processes each slot's secondaries at its
 // exclusive-scan offset.
@@ -195,8 +194,48 @@ __global__ __launch_bounds__(block_size) void generate_primaries_kernel(
         generate_primary(g, s.primaries, tid);
 }
 
+//! Counter update after the step's new tracks are initialized
+__device__ __forceinline__ void finish_initialize(StateData const& s, StepLogRef const& log)
+{
+    Counters& c = *s.counters;
+    size_type const num_new = min_of(c.num_vacancies, c.num_initializers);
+    c.num_initializers -= num_new;
+    c.num_vacancies -= num_new;
+    c.num_taken_front = 0;
+    c.num_taken_back = 0;
+    c.num_active = s.size - c.num_vacancies;
+    // pre-step clears the secondary stack
+    c.secondary_stack_size = 0;
+    StepRecord& r = log.records[*log.step_index % log.capacity];
+    r.generated = c.num_generated;
+    r.active = c.num_active;
+    c.num_generated = 0;
+}
+
+//! Whether this block is the last of its grid to get here, for every thread of
+//! the block; what the other blocks wrote before is then visible (through L2)
+//! to its first thread, and after the barrier to all. The ticket is zero again
+//! afterwards. No block waits for another.
+__device__ __forceinline__ bool last_block(size_type* ticket)
+{
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        __threadfence();
+        last = atomicAdd(ticket, size_type(1)) == gridDim.x - 1;
+        if (last)
+        {
+            *ticket = 0;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    return last;
+}
+
 __global__ __launch_bounds__(block_size) void initialize_tracks_kernel(
-    ParamsData p, StateData s)
+    ParamsData p, StateData s, StepLogRef log, size_type* ticket)
 {
     // Grid-stride over the new tracks, whose number is on the device
     Counters const c = *s.counters;
@@ -206,6 +245,9 @@ __global__ __launch_bounds__(block_size) void initialize_tracks_kernel(
     {
         init_track(p, s, c, tid);
     }
+    // Every block has read the counters when the last one gets here
+    if (last_block(ticket) && threadIdx.x == 0)
+        finish_initialize(s, log);
 }
 
 //! Track initialization with partitioned slots: the same initializers as
@@ -261,7 +303,7 @@ __global__ __launch_bounds__(block_size) void initialize_tracks_partitioned_kern
 // TrackInitAlgorithms.cc:75-95), as a per-block count, a scan of the block
 // counts and a scatter that ranks each initializer within its group. The
 // end-of-step scan scratch is free at the start of the step: block_vacant
-// holds the neutral count of each block, count[0] the total.
+// holds the neutral count of each block, block_count[0] the total.
 //---------------------------------------------------------------------------//
 __device__ __forceinline__ bool new_track_is_neutral(ParamsData const& p,
                                                      StateData const& s,
@@ -284,13 +326,14 @@ __global__ __launch_bounds__(block_size) void charge_partition_count_kernel(
         scr.block_vacant[blockIdx.x] = static_cast<size_type>(n);
 }
 
-__global__ __launch_bounds__(1024) void charge_partition_scan_kernel(ScanScratch scr)
+__global__ __launch_bounds__(1024) void charge_partition_scan_kernel(ScanScratch scr,
+                                                                     size_type num_blocks)
 {
     // Exclusive scan of the per-block neutral counts by one block
     __shared__ WideScanStorage tmp;
-    size_type const total = scan_in_place(scr.block_vacant, scr.num_blocks, 0, tmp);
+    size_type const total = scan_in_place(scr.block_vacant, num_blocks, 0, tmp);
     if (threadIdx.x == 0)
-        scr.count[0] = total;
+        scr.block_count[0] = total;
 }
 
 __global__ __launch_bounds__(block_size) void charge_partition_scatter_kernel(
@@ -312,7 +355,7 @@ __global__ __launch_bounds__(block_size) void charge_partition_scatter_kernel(
         before += warp_neutral[w];
     if (i < num_new)
     {
-        size_type const pos = neutral ? before : scr.count[0] + (i - before);
+        size_type const pos = neutral ? before : scr.block_count[0] + (i - before);
         s.init_indices[pos] = i;
     }
 }
@@ -335,35 +378,28 @@ __global__ __launch_bounds__(block_size) void clear_parents_kernel(StateData s)
         s.parents[i] = invalid_id;
 }
 
-__global__ void finish_initialize_kernel(StateData s,
-                                         StepRecord* log,
-                                         size_type log_capacity,
-                                         size_type* step_index)
+__global__ void finish_initialize_kernel(StateData s, StepLogRef log)
 {
-    Counters& c = *s.counters;
-    size_type num_new = min_of(c.num_vacancies, c.num_initializers);
-    c.num_initializers -= num_new;
-    c.num_vacancies -= num_new;
-    c.num_taken_front = 0;
-    c.num_taken_back = 0;
-    c.num_active = s.size - c.num_vacancies;
-    // pre-step clears the secondary stack
-    c.secondary_stack_size = 0;
-    StepRecord& r = log[*step_index % log_capacity];
-    r.generated = c.num_generated;
-    r.active = c.num_active;
-    c.num_generated = 0;
+    finish_initialize(s, log);
 }
 
 //---------------------------------------------------------------------------//
 // Physics actions
 //---------------------------------------------------------------------------//
-__global__ __launch_bounds__(block_size) void pre_step_kernel(ParamsData p,
-                                                              StateData s)
+//! An idle slot is written only when that changes it: what pre-step would give
+//! it, it has from its first idle step on. (The 17 to 21 bytes written for each idle
+//! slot took most of this launch's 20.5 us over 2^21 slots with a few tracks.)
+__global__ __launch_bounds__(block_size) void pre_step_kernel(ParamsData p, StateData s)
 {
     size_type slot = thread_slot();
     if (slot < s.size)
     {
+        if (s.status[slot] == status_inactive && s.post_step_action[slot] == invalid_id
+            && s.along_step_action[slot] == invalid_id
+            && s.step_length[slot] == real_type(INFINITY) && s.detector[slot] == invalid_id)
+        {
+            return;
+        }
         pre_step(p, s, slot);
         gather_pre(p, s, slot);
     }
@@ -517,42 +553,46 @@ __global__ void count_event_live_kernel(StateData s, size_type num_events)
 //---------------------------------------------------------------------------//
 // End of step: vacancies and secondaries
 //---------------------------------------------------------------------------//
+// A slot's flags byte says whether it is vacant, whether it has anything to
+// process, and how many secondaries need a new slot.
+constexpr std::uint8_t flag_vacant = 1;
+constexpr std::uint8_t flag_process = 2;
+constexpr int flag_count_shift = 2;
+
 __global__ __launch_bounds__(block_size) void locate_alive_kernel(StateData s,
                                                                   ScanScratch scr,
                                                                   bool in_place)
 {
-    __shared__ BlockScanStorage tmp;
-    size_type slot = thread_slot();
+    size_type const slot = thread_slot();
     bool vacant = false;
     size_type count = 0;
     if (slot < s.size)
     {
         locate_alive(s, slot, &vacant, &count, in_place);
-        scr.vacant[slot] = vacant;
-        scr.count[slot] = count;
+        scr.flags[slot] = static_cast<std::uint8_t>(
+            (vacant ? flag_vacant : 0)
+            | (s.status[slot] != status_inactive ? flag_process : 0)
+            | (count << flag_count_shift));
     }
-    // Block totals: vacancies with ballot/popc, counts with a block scan
-    unsigned int ballot = __ballot_sync(0xffffffffu, vacant);
-    __shared__ size_type warp_vac[block_size / 32];
+    // Vacancies and secondaries in the two halves of one word
+    size_type const sum = __reduce_add_sync(0xffffffffu, size_type(vacant) | (count << 12));
+    __shared__ size_type warp_sum[block_size / 32];
     if ((threadIdx.x & 31) == 0)
-        warp_vac[threadIdx.x >> 5] = __popc(ballot);
-    size_type total_count;
-    block_exclusive_scan(count, tmp, &total_count);
+        warp_sum[threadIdx.x >> 5] = sum;
+    __syncthreads();
     if (threadIdx.x == 0)
     {
-        size_type total_vac = 0;
+        size_type all = 0;
         for (int w = 0; w < block_size / 32; ++w)
-            total_vac += warp_vac[w];
-        scr.block_vacant[blockIdx.x] = total_vac;
-        scr.block_count[blockIdx.x] = total_count;
+            all += warp_sum[w];
+        scr.block_vacant[blockIdx.x] = all & 0xfffu;
+        scr.block_count[blockIdx.x] = all >> 12;
     }
 }
 
 __global__ __launch_bounds__(1024) void scan_blocks_kernel(StateData s,
                                                            ScanScratch scr,
-                                                           StepRecord* log,
-                                                           size_type log_capacity,
-                                                           size_type* step_index)
+                                                           StepLogRef log)
 {
     // Exclusive scan of the per-block totals by one block of 1024 threads
     __shared__ WideScanStorage tmp_vac;
@@ -577,10 +617,10 @@ __global__ __launch_bounds__(1024) void scan_blocks_kernel(StateData s,
             c.num_initializers += carry_cnt;
         }
         c.num_alive = s.size - c.num_vacancies;
-        StepRecord& r = log[*step_index % log_capacity];
+        StepRecord& r = log.records[*log.step_index % log.capacity];
         r.queued = c.num_initializers;
         r.alive = c.num_alive;
-        *step_index += 1;
+        *log.step_index += 1;
     }
 }
 
@@ -589,41 +629,21 @@ __global__ __launch_bounds__(block_size) void scatter_kernel(ParamsData p,
                                                              ScanScratch scr)
 {
     __shared__ BlockScanStorage tmp;
-    __shared__ size_type warp_vac[block_size / 32];
-    size_type slot = thread_slot();
-    bool vacant = false;
-    size_type count = 0;
-    if (slot < s.size)
-    {
-        vacant = scr.vacant[slot];
-        count = scr.count[slot];
-    }
-    // Stable position among vacant slots: ballot prefix within the warp plus
-    // preceding warps in the block plus preceding blocks
-    unsigned int ballot = __ballot_sync(0xffffffffu, vacant);
-    int const lane = threadIdx.x & 31;
-    int const warp = threadIdx.x >> 5;
-    if (lane == 0)
-        warp_vac[warp] = __popc(ballot);
-    __syncthreads();
-    size_type vac_before = 0;
-    for (int w = 0; w < warp; ++w)
-        vac_before += warp_vac[w];
-    vac_before += __popc(ballot & ((1u << lane) - 1u));
-    size_type total_count;
-    size_type count_before = block_exclusive_scan(count, tmp, &total_count);
-
-    if (slot < s.size)
+    size_type const slot = thread_slot();
+    std::uint32_t const flags = slot < s.size ? scr.flags[slot] : 0;
+    // Vacancies and secondaries before this slot in the block
+    size_type all;
+    size_type const before = block_exclusive_scan(
+        (flags & flag_vacant) | (flags >> flag_count_shift << 12), tmp, &all);
+    if (flags & flag_vacant)
+        s.vacancies[scr.block_vacant[blockIdx.x] + (before & 0xfffu)] = slot;
+    if (flags & flag_process)
     {
         Counters const c = *s.counters;
-        if (vacant)
-        {
-            s.vacancies[scr.block_vacant[blockIdx.x] + vac_before] = slot;
-        }
         if (!(c.error_flags & error_initializer_overflow))
         {
             process_secondaries(
-                p, s, c, slot, scr.block_count[blockIdx.x] + count_before);
+                p, s, c, slot, scr.block_count[blockIdx.x] + (before >> 12));
         }
     }
 }
@@ -773,6 +793,18 @@ __global__ __launch_bounds__(sort_block_size) void sort_scatter_kernel(
         s.track_slots[pos] = slot;
     }
 }
+
+//! Offsets and bins through which a sorted-range kernel visits its tracks:
+//! the action's range of the key's sort; or, for the reindexing orders
+//! (shuffle, status, particle type), every slot through the thread -> slot
+//! permutation (the shuffle's is fixed when the state is made, the others'
+//! are this step's start sort, when it runs)
+struct SlotRange
+{
+    size_type const* offsets;
+    size_type first_bin;
+    size_type end_bin;
+};
 
 //! Call f(slot) for every slot of the sorted bins [first_bin, end_bin) (or,
 //! without offsets, every slot) with a grid-stride loop: a grid of a few
@@ -935,24 +967,37 @@ __global__ __launch_bounds__(block_size) void tracking_cut_sorted_kernel(
         s, offsets, first_bin, end_bin, [&](size_type slot) { tracking_cut(p, s, slot); });
 }
 
+//! geo-boundary and tracking-cut together: a track whose crossing fails is cut
+//! in the same pass where the cut visits every slot, and left to the next step
+//! where it visits the sorted range of its action, as when the two are launched
+//! one after the other. Each is a few us of launch and first instructions when
+//! there are few tracks: together with the counters' update in the last block of
+//! the initialization, a step's two launches fewer take an FP64 calorimeter of 100
+//! electrons from 36.3 to 36.05 ms and 2000 photons from 35.76 to 35.37 ms.
+__global__ __launch_bounds__(block_size) void boundary_cut_sorted_kernel(
+    ParamsData p, StateData s, SlotRange boundary, SlotRange cut)
+{
+    bool const all = !boundary.offsets || boundary.first_bin == cut.first_bin;
+    for_each_sorted_slot(
+        s, boundary.offsets, boundary.first_bin, boundary.end_bin, [&](size_type slot) {
+            boundary_cross(p, s, slot);
+            if (all)
+                tracking_cut(p, s, slot);
+        });
+    if (!all)
+    {
+        for_each_sorted_slot(s, cut.offsets, cut.first_bin, cut.end_bin, [&](size_type slot) {
+            tracking_cut(p, s, slot);
+        });
+    }
+}
+
 //! Bin offsets written by the sort for a key
 inline size_type* sort_offsets(LaunchContext const& ctx, SortKey key)
 {
     std::size_t const table = std::size_t(ctx.sort.num_bins) + 1;
     return ctx.state.action_offsets + (key == SortKey::step_limit ? table : 0);
 }
-
-//! Offsets and bins through which a sorted-range kernel visits its tracks:
-//! the action's range of the key's sort; or, for the reindexing orders
-//! (shuffle, status, particle type), every slot through the thread -> slot
-//! permutation (the shuffle's is fixed when the state is made, the others'
-//! are this step's start sort, when it runs)
-struct SlotRange
-{
-    size_type const* offsets;
-    size_type first_bin;
-    size_type end_bin;
-};
 
 inline SlotRange
 slot_range(LaunchContext const& ctx, SortKey key, size_type first_bin, size_type end_bin)
@@ -1001,13 +1046,12 @@ void launch_initialize_tracks(LaunchContext const& ctx, cudaStream_t stream)
         unsigned int const nb = num_blocks_for(ctx.state.size);
         charge_partition_count_kernel<<<nb, block_size, 0, stream>>>(
             ctx.params, ctx.state, ctx.scratch);
-        charge_partition_scan_kernel<<<1, 1024, 0, stream>>>(ctx.scratch);
+        charge_partition_scan_kernel<<<1, 1024, 0, stream>>>(ctx.scratch, nb);
         charge_partition_scatter_kernel<<<nb, block_size, 0, stream>>>(
             ctx.params, ctx.state, ctx.scratch);
         initialize_tracks_charge_kernel<<<ctx.range_blocks, block_size, 0, stream>>>(
             ctx.params, ctx.state);
-        finish_initialize_kernel<<<1, 1, 0, stream>>>(
-            ctx.state, ctx.log, ctx.log_capacity, ctx.step_index);
+        finish_initialize_kernel<<<1, 1, 0, stream>>>(ctx.state, ctx.log);
         clear_parents_kernel<<<ctx.range_blocks, block_size, 0, stream>>>(ctx.state);
         return;
     }
@@ -1017,14 +1061,11 @@ void launch_initialize_tracks(LaunchContext const& ctx, cudaStream_t stream)
                                                block_size,
                                                0,
                                                stream>>>(ctx.params, ctx.state);
+        finish_initialize_kernel<<<1, 1, 0, stream>>>(ctx.state, ctx.log);
+        return;
     }
-    else
-    {
-        initialize_tracks_kernel<<<ctx.range_blocks, block_size, 0, stream>>>(ctx.params,
-                                                                            ctx.state);
-    }
-    finish_initialize_kernel<<<1, 1, 0, stream>>>(
-        ctx.state, ctx.log, ctx.log_capacity, ctx.step_index);
+    initialize_tracks_kernel<<<ctx.range_blocks, block_size, 0, stream>>>(
+        ctx.params, ctx.state, ctx.log, ctx.scratch.ticket);
 }
 
 void launch_pre_step(LaunchContext const& ctx, cudaStream_t stream)
@@ -1135,6 +1176,16 @@ void launch_tracking_cut(LaunchContext const& ctx, cudaStream_t stream)
         p, ctx.state, r.offsets, r.first_bin, r.end_bin);
 }
 
+void launch_boundary_cut(LaunchContext const& ctx, cudaStream_t stream)
+{
+    ParamsData const& p = ctx.params;
+    boundary_cut_sorted_kernel<<<ctx.range_blocks, block_size, 0, stream>>>(
+        p,
+        ctx.state,
+        slot_range(ctx, SortKey::step_limit, p.action_boundary, p.action_boundary + 1),
+        slot_range(ctx, SortKey::step_limit, p.action_tracking_cut, p.action_tracking_cut + 1));
+}
+
 void launch_calo_tally(LaunchContext const& ctx, cudaStream_t stream)
 {
     unsigned int const nb = num_blocks_for(ctx.state.size);
@@ -1146,18 +1197,17 @@ void launch_calo_tally(LaunchContext const& ctx, cudaStream_t stream)
         hits_scan_kernel<<<1, 1024, 0, stream>>>(
             ctx.state, ctx.hit_block_offsets, nb, ctx.hits.capacity);
         hits_scatter_kernel<<<nb, block_size, 0, stream>>>(
-            ctx.params, ctx.state, ctx.hits, ctx.hit_block_offsets, ctx.step_index);
+            ctx.params, ctx.state, ctx.hits, ctx.hit_block_offsets, ctx.log.step_index);
     }
 }
 
 void launch_extend_from_secondaries(LaunchContext const& ctx, cudaStream_t stream)
 {
-    unsigned int nb = num_blocks_for(ctx.state.size);
-    locate_alive_kernel<<<nb, block_size, 0, stream>>>(
-        ctx.state, ctx.scratch, !partitions_by_charge(ctx.params.track_order));
-    scan_blocks_kernel<<<1, 1024, 0, stream>>>(
-        ctx.state, ctx.scratch, ctx.log, ctx.log_capacity, ctx.step_index);
-    scatter_kernel<<<nb, block_size, 0, stream>>>(ctx.params, ctx.state, ctx.scratch);
+    ScanScratch const& scr = ctx.scratch;
+    locate_alive_kernel<<<scr.num_blocks, block_size, 0, stream>>>(
+        ctx.state, scr, !partitions_by_charge(ctx.params.track_order));
+    scan_blocks_kernel<<<1, 1024, 0, stream>>>(ctx.state, scr, ctx.log);
+    scatter_kernel<<<scr.num_blocks, block_size, 0, stream>>>(ctx.params, ctx.state, scr);
 }
 
 int persistent_along_blocks(int threads_per_block)
@@ -1253,12 +1303,12 @@ void launch_sort_tracks(LaunchContext const& ctx, SortKey key, cudaStream_t stre
 //---------------------------------------------------------------------------//
 // Extend-from-secondaries with library-owned scratch
 //---------------------------------------------------------------------------//
-// The three extend-from-secondaries kernels need 5 bytes of scratch per
-// track slot plus 8 bytes per block. This variant takes that scratch from
-// one array compiled into the library instead of the stepper's allocation,
-// for callers that may not allocate device memory at all. Layout for n
-// slots and b = ceil(n / block_size) blocks, each part 256-byte aligned:
-//   block_vacant[b] | block_count[b] | count[n] | vacant[n]
+// The three extend-from-secondaries kernels need a byte of scratch per track slot
+// plus 8 bytes per block. This variant takes that scratch from one array compiled
+// into the library instead of the stepper's allocation, for callers that may not
+// allocate device memory at all. Layout for n slots and b = ceil(n / block_size)
+// blocks, each part 256-byte aligned:
+//   block_vacant[b] | block_count[b] | flags[n]
 namespace
 {
 constexpr std::size_t align_256(std::size_t bytes)
@@ -1269,11 +1319,10 @@ constexpr std::size_t align_256(std::size_t bytes)
 constexpr std::size_t static_scratch_bytes(std::size_t n)
 {
     std::size_t const b = (n + block_size - 1) / block_size;
-    return 2 * align_256(b * sizeof(size_type))
-           + align_256(n * sizeof(size_type)) + align_256(n);
+    return 2 * align_256(b * sizeof(size_type)) + align_256(n);
 }
 
-// 659,456 bytes for 131,072 track slots
+// 135,168 bytes for 131,072 track slots
 constexpr std::size_t static_scratch_capacity
     = static_scratch_bytes(static_scratch_max_slots);
 
@@ -1330,22 +1379,20 @@ void launch_extend_from_secondaries_static(LaunchContext const& ctx,
     unsigned char* base = static_scratch_for_current_device();
     unsigned int const nb = num_blocks_for(n);
     std::size_t const block_part = align_256(std::size_t(nb) * sizeof(size_type));
-    std::size_t const count_part = align_256(std::size_t(n) * sizeof(size_type));
 
-    // Nothing is cleared: locate_alive_kernel writes vacant/count for every
-    // slot and both totals for every block before the scan and scatter
-    // kernels read them, so the previous call's contents are never used
+    // Nothing is cleared: locate_alive_kernel writes the flags of every slot
+    // and both totals of every block before it and the scatter kernel read
+    // them, so the previous call's contents are never used
     ScanScratch scr;
     scr.block_vacant = reinterpret_cast<size_type*>(base);
     scr.block_count = reinterpret_cast<size_type*>(base + block_part);
-    scr.count = reinterpret_cast<size_type*>(base + 2 * block_part);
-    scr.vacant = base + 2 * block_part + count_part;
+    scr.flags = base + 2 * block_part;
+    scr.ticket = ctx.scratch.ticket;
     scr.num_blocks = nb;
 
     locate_alive_kernel<<<nb, block_size, 0, stream>>>(
         ctx.state, scr, !partitions_by_charge(ctx.params.track_order));
-    scan_blocks_kernel<<<1, 1024, 0, stream>>>(
-        ctx.state, scr, ctx.log, ctx.log_capacity, ctx.step_index);
+    scan_blocks_kernel<<<1, 1024, 0, stream>>>(ctx.state, scr, ctx.log);
     scatter_kernel<<<nb, block_size, 0, stream>>>(ctx.params, ctx.state, scr);
 }
 

@@ -16,13 +16,22 @@ struct StepRecord
     size_type alive;
 };
 
+//! Step log (ring buffer) and the device-resident step counter
+struct StepLogRef
+{
+    StepRecord* records;
+    size_type capacity;
+    size_type* step_index;
+};
+
 //! Scratch for the end-of-step compaction: per-block totals and offsets
 struct ScanScratch
 {
     size_type* block_vacant;  //!< [num_blocks]
     size_type* block_count;  //!< [num_blocks]
-    std::uint8_t* vacant;  //!< [num_slots]
-    size_type* count;  //!< [num_slots]
+    std::uint8_t* flags;  //!< [num_slots]
+    //! Blocks done of the initialization (zero between launches)
+    size_type* ticket;
     size_type num_blocks;
 };
 
@@ -117,9 +126,7 @@ struct LaunchContext
     //! ones the highest (per-track random streams only), so that each
     //! along-step kernel's sorted range covers mostly contiguous slots
     bool partition_slots;
-    StepRecord* log;  //!< Step log (ring buffer)
-    size_type log_capacity;
-    size_type* step_index;  //!< Device-resident step counter
+    StepLogRef log;
     //! Step output (disabled: zero capacity) and its per-block hit counts
     StepHitsRef hits;
     size_type* hit_block_offsets;  //!< [num_blocks_for(size)]
@@ -146,6 +153,8 @@ void launch_interact(LaunchContext const& ctx,
                      cudaStream_t stream);
 void launch_boundary(LaunchContext const& ctx, cudaStream_t stream);
 void launch_tracking_cut(LaunchContext const& ctx, cudaStream_t stream);
+//! Both of the above in one launch
+void launch_boundary_cut(LaunchContext const& ctx, cudaStream_t stream);
 //! SimpleCalo tally and, when enabled, the step output (step-gather-post)
 void launch_calo_tally(LaunchContext const& ctx, cudaStream_t stream);
 void launch_extend_from_secondaries(LaunchContext const& ctx,

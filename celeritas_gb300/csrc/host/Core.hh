@@ -200,7 +200,7 @@ class CoreState
     event_detector_energy_deposition(size_type first, size_type n, bool clear);
     //! Read the step log entries [first, first + n)
     std::vector<StepRecord> step_log(size_type first, size_type n) const;
-    size_type log_capacity() const { return ctx_.log_capacity; }
+    size_type log_capacity() const { return ctx_.log.capacity; }
 
     //! Collect the hits of every step (StepCollector with DetectorSteps):
     //! the selected data of each track step in a detector volume, dropping

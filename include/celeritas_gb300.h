@@ -488,7 +488,7 @@ int gbx_device_allocations(unsigned long long* count);
  * (an allocation there would bypass the pool's accounting, may synchronise
  * the device, and can fail once the pool has claimed the memory).
  *
- * - The scratch is 659,456 bytes and fits steppers of at most
+ * - The scratch is 135,168 bytes and fits steppers of at most
  *   GBX_STATIC_SCRATCH_MAX_SLOTS track slots; larger ones are rejected with
  *   an error and nothing is launched.
  * - The array's device address is looked up (cudaGetSymbolAddress) once
