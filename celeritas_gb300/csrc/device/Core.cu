@@ -497,7 +497,8 @@ CoreState::CoreState(CoreParams const& params,
     std::size_t o_aoff = L.reserve(4 * 2 * std::size_t(num_bins + 1));
     std::size_t o_shist = L.reserve(4 * std::size_t(num_bins) * sort_blocks);
     std::size_t o_stot = L.reserve(4 * std::size_t(num_bins));
-    std::size_t o_work = L.reserve(sizeof(size_type));
+    std::size_t o_work = L.reserve(3 * sizeof(size_type));
+    std::size_t o_charged = arr(4);
     std::size_t o_log = L.reserve(sizeof(StepRecord) * log_cap);
     std::size_t o_stepidx = L.reserve(sizeof(size_type));
 
@@ -662,7 +663,9 @@ CoreState::CoreState(CoreParams const& params,
     ctx_.sort.material_actions[0] = invalid_id;
     ctx_.sort.material_actions[1] = invalid_id;
     ctx_.sort.track_order = params.host().scalars.track_order;
-    ctx_.work_counter = static_cast<size_type*>(at(o_work));
+    ctx_.along_work.counter = static_cast<size_type*>(at(o_work));
+    ctx_.along_work.offsets = ctx_.along_work.counter + 1;
+    ctx_.along_work.slots = static_cast<size_type*>(at(o_charged));
     // Persistent charged along-step: on by default in the mixed-precision
     // build, where it outruns the one-thread-per-track kernel; in FP64 the
     // diverged FP64 multiple-scattering code makes it slower
@@ -675,6 +678,7 @@ CoreState::CoreState(CoreParams const& params,
         GBX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         ctx_.range_blocks = std::min<unsigned int>(
             (n + block_size - 1) / block_size, 8u * static_cast<unsigned int>(sms));
+        ctx_.num_sms = static_cast<size_type>(sms);
     }
     ctx_.persistent_blocks = sizeof(real_type) < sizeof(double)
                                  ? persistent_along_blocks(ctx_.along_block_size)

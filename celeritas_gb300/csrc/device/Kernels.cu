@@ -828,6 +828,7 @@ __global__ __launch_bounds__(sort_block_size) void sort_scatter_kernel(
 //! are this step's start sort, when it runs)
 struct SlotRange
 {
+    size_type const* slots;
     size_type const* offsets;
     size_type first_bin;
     size_type end_bin;
@@ -880,24 +881,75 @@ __device__ __forceinline__ void for_each_sorted_slot(StateData const& s,
 #endif
 constexpr int along_block_large = 512;
 
-template<AlongKind K, int Threads = block_size>
-__global__ GBX_ALONG_BOUNDS(Threads, K == AlongKind::charged ? GBX_ALONG_MIN_BLOCKS : 1) void
-along_step_sorted_kernel(ParamsData p,
-                         StateData s,
-                         size_type const* offsets,
-                         size_type first_bin,
-                         size_type end_bin)
+//! Threads on every SM over which few tracks are spread
+constexpr int spread_threads = 256;
+
+//! Whether 'count' tracks are few enough to be spread over the warps of the first
+//! 'blocks' blocks (which all fit on the GPU), and the one that this thread gets.
+//! Tracks in a field take paths and times of their own: one that curls up for a
+//! million cycles alone took up to 1.9 million beside 31 others. A warp therefore
+//! gets a second track only when every warp has one, neighbours in different SMs.
+//! From 32 tracks a warp on, one after the other is the better order (coalesced
+//! access). 650 particles in the CMS-like detector in 2^21 slots 377 -> 358 ms with
+//! the launch settings found for it and 571 -> 393 ms with the default (persistent)
+//! ones, an FP64 event of 20 there 477 -> 458 ms; with at most 4 or 16 tracks a warp
+//! the first took 373 and 364 ms.
+__device__ __forceinline__ bool
+spread_track(size_type count, size_type blocks, size_type* index)
 {
-    begin_dependent();
-    for_each_sorted_slot(s, offsets, first_bin, end_bin, [&](size_type slot) {
-        along_step_impl<K>(p, s, slot);
-    });
+    size_type const warps = blocks * (blockDim.x >> 5);
+    if (count > warps * 31)
+        return false;
+    size_type const lane = threadIdx.x & 31u;
+    *index = blockIdx.x < blocks ? lane * warps + (threadIdx.x >> 5) * blocks + blockIdx.x
+                                 : count;
+    return true;
 }
 
-__global__ void clear_counter_kernel(size_type* counter)
+template<AlongKind K, int Threads = block_size>
+__global__ GBX_ALONG_BOUNDS(Threads, K == AlongKind::charged ? GBX_ALONG_MIN_BLOCKS : 1) void
+along_step_sorted_kernel(ParamsData p, StateData s, SlotRange range, size_type spread_blocks)
 {
     begin_dependent();
-    *counter = 0;
+    size_type const first = range.offsets ? range.offsets[range.first_bin] : 0;
+    size_type const count = range.offsets ? range.offsets[range.end_bin] - first : s.size;
+    size_type stride = gridDim.x * blockDim.x;
+    size_type index = thread_slot();
+    if (spread_blocks && spread_track(count, spread_blocks, &index))
+        stride = count;
+    for (; index < count; index += stride)
+    {
+        along_step_impl<K>(p, s, range.offsets ? range.slots[first + index] : index);
+    }
+}
+
+//! Before a charged along-step in a field: no track claimed, none listed
+__global__ void clear_along_work_kernel(AlongWork work)
+{
+    begin_dependent();
+    *work.counter = 0;
+    work.offsets[1] = 0;
+}
+
+//! List the tracks of the charged along-step where the state is not sorted by
+//! it, in no particular order
+__global__ __launch_bounds__(block_size) void
+list_charged_kernel(ParamsData p, StateData s, AlongWork work)
+{
+    begin_dependent();
+    size_type const slot = thread_slot();
+    bool const charged = slot < s.size && is_track_valid(s.status[slot])
+                         && s.along_step_action[slot] == p.action_along_step;
+    unsigned int const ballot = __ballot_sync(0xffffffffu, charged);
+    if (!ballot)
+        return;
+    unsigned int const lane = threadIdx.x & 31u;
+    size_type base = 0;
+    if (lane == 0)
+        base = atomicAdd(work.offsets + 1, size_type(__popc(ballot)));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (charged)
+        work.slots[base + __popc(ballot & ((1u << lane) - 1u))] = slot;
 }
 
 //! Charged along-step in a uniform field over the sorted charged range, as
@@ -909,16 +961,13 @@ __global__ void clear_counter_kernel(size_type* counter)
 //! the same sequence of operations as along_step_impl.
 template<int Threads>
 __global__ GBX_ALONG_BOUNDS(Threads, 1) void along_charged_persistent_kernel(
-    ParamsData p,
-    StateData s,
-    size_type const* offsets,
-    size_type first_bin,
-    size_type end_bin,
-    size_type* work_counter)
+    ParamsData p, StateData s, SlotRange range, size_type* work_counter)
 {
     begin_dependent();
-    size_type const first = offsets ? offsets[first_bin] : 0;
-    size_type const count = offsets ? offsets[end_bin] - first : s.size;
+    size_type const first = range.offsets[range.first_bin];
+    size_type const count = range.offsets[range.end_bin] - first;
+    size_type spread_index = count;
+    bool const spread = spread_track(count, gridDim.x, &spread_index);
     unsigned int const lane = threadIdx.x & 31u;
     FieldOptions const& opt = p.field_options;
     FieldPropagation<false> fp(opt, UniformFieldEquation{});
@@ -928,18 +977,23 @@ __global__ GBX_ALONG_BOUNDS(Threads, 1) void along_charged_persistent_kernel(
     {
         if (!have)
         {
-            // Claim the next track for every lane that needs one
-            unsigned int const need = __activemask();
-            unsigned int const rank = __popc(need & ((1u << lane) - 1u));
-            unsigned int const leader = __ffs(need) - 1;
-            size_type base = 0;
-            if (lane == leader)
-                base = atomicAdd(work_counter, size_type(__popc(need)));
-            base = __shfl_sync(need, base, leader);
-            size_type const idx = base + rank;
+            size_type idx = spread_index;
+            spread_index = count;
+            if (!spread)
+            {
+                // Claim the next track for every lane that needs one
+                unsigned int const need = __activemask();
+                unsigned int const rank = __popc(need & ((1u << lane) - 1u));
+                unsigned int const leader = __ffs(need) - 1;
+                size_type base = 0;
+                if (lane == leader)
+                    base = atomicAdd(work_counter, size_type(__popc(need)));
+                base = __shfl_sync(need, base, leader);
+                idx = base + rank;
+            }
             if (idx >= count)
                 break;
-            slot = offsets ? s.track_slots[first + idx] : idx;
+            slot = range.slots[first + idx];
             bool charged;
             double start_safety;
             if (!along_prologue<AlongKind::charged>(p, s, slot, &charged, &start_safety))
@@ -1045,11 +1099,17 @@ slot_range(LaunchContext const& ctx, SortKey key, size_type first_bin, size_type
     if (reindexes_all(order))
     {
         bool const permuted = order == track_order_reindex_shuffle || ctx.sort_enabled;
-        return {permuted ? sort_offsets(ctx, SortKey::start) : nullptr, 0, ctx.sort.num_bins};
+        return {ctx.state.track_slots,
+                permuted ? sort_offsets(ctx, SortKey::start) : nullptr,
+                0,
+                ctx.sort.num_bins};
     }
     bool const sorts = key == SortKey::along_step ? sorts_along_step(order)
                                                   : sorts_step_limit(order);
-    return {sorts && ctx.sort_enabled ? sort_offsets(ctx, key) : nullptr, first_bin, end_bin};
+    return {ctx.state.track_slots,
+            sorts && ctx.sort_enabled ? sort_offsets(ctx, key) : nullptr,
+            first_bin,
+            end_bin};
 }
 
 }  // namespace
@@ -1161,43 +1221,51 @@ void launch_along_step(LaunchContext const& ctx,
     size_type cfirst, cend, nfirst, nend;
     along_bins(ctx.sort, p.action_along_step, &cfirst, &cend);
     along_bins(ctx.sort, p.action_along_step_neutral, &nfirst, &nend);
-    SlotRange const cr = slot_range(ctx, SortKey::along_step, cfirst, cend);
-    SlotRange const nr = slot_range(ctx, SortKey::along_step, nfirst, nend);
-    size_type const* offsets = cr.offsets;
-    cfirst = cr.first_bin;
-    cend = cr.end_bin;
-    nfirst = nr.first_bin;
-    nend = nr.end_bin;
     if (action == invalid_id || action == p.action_along_step)
     {
+        SlotRange range = slot_range(ctx, SortKey::along_step, cfirst, cend);
         bool const large = abs > static_cast<unsigned int>(block_size);
+        unsigned int blocks = cnb;
+        size_type spread_blocks = 0;
+        if (p.has_field)
+        {
+            launch(clear_along_work_kernel, 1, 1, 0, stream, ctx.along_work);
+            if (!range.offsets || reindexes_all(p.track_order))
+            {
+                launch(list_charged_kernel, nb, block_size, 0, stream, p, ctx.state,
+                       ctx.along_work);
+                range = {ctx.along_work.slots, ctx.along_work.offsets, 0, 1};
+            }
+            spread_blocks = ctx.num_sms * max_of(1u, spread_threads / abs);
+            blocks = max_of<unsigned int>(blocks, spread_blocks);
+        }
         if (p.has_field && ctx.persistent_blocks > 0)
         {
-            launch(clear_counter_kernel, 1, 1, 0, stream, ctx.work_counter);
             if (large)
                 launch(along_charged_persistent_kernel<along_block_large>,
-                       ctx.persistent_blocks, abs, 0, stream, p, ctx.state, offsets,
-                       cfirst, cend, ctx.work_counter);
+                       ctx.persistent_blocks, abs, 0, stream, p, ctx.state, range,
+                       ctx.along_work.counter);
             else
                 launch(along_charged_persistent_kernel<block_size>,
-                       ctx.persistent_blocks, abs, 0, stream, p, ctx.state, offsets,
-                       cfirst, cend, ctx.work_counter);
+                       ctx.persistent_blocks, abs, 0, stream, p, ctx.state, range,
+                       ctx.along_work.counter);
         }
         else if (large)
         {
-            launch(along_step_sorted_kernel<AlongKind::charged, along_block_large>, cnb,
-                   abs, 0, stream, p, ctx.state, offsets, cfirst, cend);
+            launch(along_step_sorted_kernel<AlongKind::charged, along_block_large>, blocks,
+                   abs, 0, stream, p, ctx.state, range, spread_blocks);
         }
         else
         {
-            launch(along_step_sorted_kernel<AlongKind::charged>, cnb, abs, 0, stream, p,
-                   ctx.state, offsets, cfirst, cend);
+            launch(along_step_sorted_kernel<AlongKind::charged>, blocks, abs, 0, stream, p,
+                   ctx.state, range, spread_blocks);
         }
     }
     if (action == invalid_id || action == p.action_along_step_neutral)
     {
-        launch(along_step_sorted_kernel<AlongKind::neutral>, ctx.range_blocks,
-               block_size, 0, stream, p, ctx.state, offsets, nfirst, nend);
+        SlotRange const range = slot_range(ctx, SortKey::along_step, nfirst, nend);
+        launch(along_step_sorted_kernel<AlongKind::neutral>, ctx.range_blocks, block_size, 0,
+               stream, p, ctx.state, range, 0u);
     }
 }
 

@@ -105,22 +105,30 @@ enum ErrorFlag : size_type
 constexpr int block_size = 256;
 constexpr int sort_block_size = 1024;
 
+//! Work of the charged along-step in a field
+struct AlongWork
+{
+    size_type* counter;  //!< Next track of the persistent kernel
+    size_type* offsets;  //!< [2]: zero, length of the list
+    size_type* slots;  //!< [num_slots] List of the charged tracks
+};
+
 struct LaunchContext
 {
     ParamsData params;
     StateData state;
     ScanScratch scratch;
     SortScratch sort;
-    //! Grid of the persistent charged along-step kernel (0: not used) and
-    //! its device work counter
+    //! Grid of the persistent charged along-step kernel (0: not used)
     int persistent_blocks;
-    size_type* work_counter;
+    AlongWork along_work;
     //! Tuning: threads per block of the charged along-step kernels (at most
     //! block_size) and whether the action sorts run this step
     int along_block_size;
     //! Grid of the short sorted-range kernels (grid-stride loops): a few
     //! blocks per SM, at most one block per block_size slots
     unsigned int range_blocks;
+    size_type num_sms;
     bool sort_enabled;
     //! Tuning: new charged tracks take the lowest vacant slots and neutral
     //! ones the highest (per-track random streams only), so that each
