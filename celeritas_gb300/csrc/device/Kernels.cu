@@ -906,21 +906,58 @@ spread_track(size_type count, size_type blocks, size_type* index)
     return true;
 }
 
-template<AlongKind K, int Threads = block_size>
+//! Spread: see spread_track(), over the first 'spread_blocks' blocks; up to
+//! 'warp_tracks' tracks are left to along_charged_warp_kernel
+template<AlongKind K, int Threads = block_size, bool Spread = false>
 __global__ GBX_ALONG_BOUNDS(Threads, K == AlongKind::charged ? GBX_ALONG_MIN_BLOCKS : 1) void
-along_step_sorted_kernel(ParamsData p, StateData s, SlotRange range, size_type spread_blocks)
+along_step_sorted_kernel(ParamsData p,
+                         StateData s,
+                         SlotRange range,
+                         size_type spread_blocks,
+                         size_type warp_tracks)
 {
     begin_dependent();
     size_type const first = range.offsets ? range.offsets[range.first_bin] : 0;
     size_type const count = range.offsets ? range.offsets[range.end_bin] - first : s.size;
     size_type stride = gridDim.x * blockDim.x;
     size_type index = thread_slot();
-    if (spread_blocks && spread_track(count, spread_blocks, &index))
-        stride = count;
+    if constexpr (Spread)
+    {
+        if (count <= warp_tracks)
+            return;
+        if (spread_track(count, spread_blocks, &index))
+            stride = count;
+    }
     for (; index < count; index += stride)
     {
         along_step_impl<K>(p, s, range.offsets ? range.slots[first + index] : index);
     }
+}
+
+//! FP64 charged along-step in a field of at most 'warp_tracks' tracks, the warps of
+//! this grid: each runs one, lane 0 the track and the others its Runge-Kutta steps
+//! with it (warp_step). Fewer warps than a block of 8 on every SM are worse also where
+//! the FP64 units are shared (300 electrons in the calorimeter with at most 1, 2, 4, 8
+//! tracks per SM: 239, 237, 234, 233 ms). A kernel of its own: in one with
+//! along_step_sorted_kernel it makes that one 4% slower (233 against 224.5 ms).
+__global__ __launch_bounds__(block_size, 1) void along_charged_warp_kernel(
+    ParamsData p, StateData s, SlotRange range, size_type warp_tracks)
+{
+    begin_dependent();
+    size_type const first = range.offsets[range.first_bin];
+    size_type const count = range.offsets[range.end_bin] - first;
+    if (count > warp_tracks)
+        return;
+    size_type const track = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    if (track >= count)
+        return;
+    if ((threadIdx.x & 31u) != 0)
+    {
+        help_field_warp();
+        return;
+    }
+    along_step_impl<AlongKind::charged, true>(p, s, range.slots[first + track]);
+    end_field_warp();
 }
 
 //! Before a charged along-step in a field: no track claimed, none listed
@@ -1227,6 +1264,7 @@ void launch_along_step(LaunchContext const& ctx,
         bool const large = abs > static_cast<unsigned int>(block_size);
         unsigned int blocks = cnb;
         size_type spread_blocks = 0;
+        size_type warp_tracks = 0;
         if (p.has_field)
         {
             launch(clear_along_work_kernel, 1, 1, 0, stream, ctx.along_work);
@@ -1238,6 +1276,14 @@ void launch_along_step(LaunchContext const& ctx,
             }
             spread_blocks = ctx.num_sms * max_of(1u, spread_threads / abs);
             blocks = max_of<unsigned int>(blocks, spread_blocks);
+            // One track per warp of a block on every SM; the persistent kernel
+            // takes all its tracks itself
+            if (sizeof(real_type) == sizeof(double) && ctx.persistent_blocks == 0)
+            {
+                warp_tracks = ctx.num_sms * (block_size / 32);
+                launch(along_charged_warp_kernel, ctx.num_sms, block_size, 0, stream, p,
+                       ctx.state, range, warp_tracks);
+            }
         }
         if (p.has_field && ctx.persistent_blocks > 0)
         {
@@ -1250,22 +1296,24 @@ void launch_along_step(LaunchContext const& ctx,
                        ctx.persistent_blocks, abs, 0, stream, p, ctx.state, range,
                        ctx.along_work.counter);
         }
-        else if (large)
-        {
-            launch(along_step_sorted_kernel<AlongKind::charged, along_block_large>, blocks,
-                   abs, 0, stream, p, ctx.state, range, spread_blocks);
-        }
         else
         {
-            launch(along_step_sorted_kernel<AlongKind::charged>, blocks, abs, 0, stream, p,
-                   ctx.state, range, spread_blocks);
+            auto* kernel
+                = large ? (p.has_field
+                               ? along_step_sorted_kernel<AlongKind::charged, along_block_large, true>
+                               : along_step_sorted_kernel<AlongKind::charged, along_block_large>)
+                        : (p.has_field
+                               ? along_step_sorted_kernel<AlongKind::charged, block_size, true>
+                               : along_step_sorted_kernel<AlongKind::charged>);
+            launch(kernel, blocks, abs, 0, stream, p, ctx.state, range, spread_blocks,
+                   warp_tracks);
         }
     }
     if (action == invalid_id || action == p.action_along_step_neutral)
     {
         SlotRange const range = slot_range(ctx, SortKey::along_step, nfirst, nend);
         launch(along_step_sorted_kernel<AlongKind::neutral>, ctx.range_blocks, block_size, 0,
-               stream, p, ctx.state, range, 0u);
+               stream, p, ctx.state, range, 0u, 0u);
     }
 }
 

@@ -434,9 +434,10 @@ GBX_FUNCTION void along_epilogue(ParamsData const& p,
 }
 
 //! The whole along-step of one slot (PropagationApplier between the MSC
-//! step limit and the MSC applier, then time, energy loss, track update)
-template<AlongKind K>
-GBX_FUNCTION void along_step_impl(ParamsData const& p, StateData const& s, size_type slot)
+//! step limit and the MSC applier, then time, energy loss, track update).
+//! Warp: see FieldPropagation
+template<AlongKind K, bool Warp = false>
+GBX_FORCEINLINE void along_step_impl(ParamsData const& p, StateData const& s, size_type slot)
 {
     bool charged;
     double start_safety;
@@ -450,7 +451,7 @@ GBX_FUNCTION void along_step_impl(ParamsData const& p, StateData const& s, size_
         if (charged && p.has_field)
         {
             FieldOptions const& opt = p.field_options;
-            FieldPropagation<> fp(opt, UniformFieldEquation{});
+            FieldPropagation<true, Warp> fp(opt, UniformFieldEquation{});
             field_setup(p, s, slot, geo, &fp, start_safety);
             do
             {

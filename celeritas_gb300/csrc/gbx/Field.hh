@@ -92,16 +92,15 @@ struct FixedFieldEquation
     }
 };
 
-//! Dormand-Prince 5(4) step: the stages and the end state when made; the error
+//! Dormand-Prince 5(4) step: the stages and the end state when taken; the error
 //! estimate and Shampine's midpoint where the driver asks for them
 template<class Equation>
 class DormandPrinceStep
 {
   public:
-    GBX_FORCEINLINE
-    DormandPrinceStep(Equation const& rhs, double step, OdeState const& beg_state)
-        : step_(step)
+    GBX_FORCEINLINE void take(Equation const& rhs, double step, OdeState const& beg_state)
     {
+        step_ = step;
         using R = double;
         constexpr R a11 = 0.2;
         constexpr R a21 = 0.075;
@@ -209,6 +208,206 @@ class DormandPrinceStep
     OdeState end_;
 };
 
+//! A step taken by a warp: its end, and the two numbers by which the driver
+//! accepts it
+struct WarpStep
+{
+    OdeState end;
+    double dchord;  //!< Distance of the midpoint from the chord, if asked for
+    double rel_err_sq;  //!< Relative squared error, unless the chord is too far
+    bool active;  //!< A step was taken
+};
+
+#if defined(__CUDACC__)
+//! Coefficients of the step: a11, a21 a22, a31..a33, a41..a44, a51..a55, a61 a63..a66;
+//! d71 d73..d77; c71 c73..c77 (names of DormandPrinceStep)
+static __device__ double const warp_step_coefficients[32] = {
+    0.2,
+    0.075,
+    0.225,
+    44 / double(45),
+    -56 / double(15),
+    32 / double(9),
+    19372 / double(6561),
+    -25360 / double(2187),
+    64448 / double(6561),
+    -212 / double(729),
+    9017 / double(3168),
+    -355 / double(33),
+    46732 / double(5247),
+    49 / double(176),
+    -5103 / double(18656),
+    35 / double(384),
+    500 / double(1113),
+    125 / double(192),
+    -2187 / double(6784),
+    11 / double(84),
+    35 / double(384) - 5179 / double(57600),
+    500 / double(1113) - 7571 / double(16695),
+    125 / double(192) - 393 / double(640),
+    -2187 / double(6784) + 92097 / double(339200),
+    11 / double(84) - 187 / double(2100),
+    -1 / double(40),
+    double(6025192743.) / double(30085553152.),
+    double(51252292925.) / double(65400821598.),
+    double(-2691868925.) / double(45128329728.),
+    double(187940372067.) / double(1594534317056.),
+    double(-1776094331.) / double(19743644256.),
+    double(11237099.) / double(235043384.)};
+
+//! One Dormand-Prince step of one track by the 32 lanes of its warp, which all call
+//! this: lane 0 with the track's arguments, the others with 'active' alone looked
+//! at in lane 0 (no step, and the helpers are done, if it is false).
+//!
+//! On GB300 an FP64 instruction takes its warp 64 cycles whatever its lanes do, and
+//! none overlaps another. With few tracks, each in a warp of its own, three lanes
+//! hold the position, three the momentum and three the midpoint's position, so
+//! that each of the 26 + 6 accumulations is one instruction instead of six, each
+//! evaluation 8 instead of 19, and the 32 products of the step and a coefficient
+//! one. Every lane does the operations of DormandPrinceStep, rel_err_sq and
+//! distance_chord for its component, so the results are theirs bit for bit. An event
+//! of 20 particles in the CMS-like detector 458 -> 363 ms, 7 with detector hits 77 -> 65
+//! ms, 300 electrons in the calorimeter 230 -> 224.5 ms.
+__device__ __noinline__ WarpStep warp_step(
+    bool active, UniformFieldEquation rhs, double step, OdeState beg, double chord_limit)
+{
+    auto from = [](double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); };
+    WarpStep result;
+    __syncwarp();
+    result.active = __shfl_sync(0xffffffffu, int(active), 0);
+    if (!result.active)
+        return result;
+    step = from(step, 0);
+    chord_limit = from(chord_limit, 0);
+    rhs.coeffi = from(rhs.coeffi, 0);
+    rhs.field = {from(rhs.field.x, 0), from(rhs.field.y, 0), from(rhs.field.z, 0)};
+    rhs.map = reinterpret_cast<RZMapData const*>(
+        __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(rhs.map), 0));
+    beg.pos = {from(beg.pos.x, 0), from(beg.pos.y, 0), from(beg.pos.z, 0)};
+    beg.mom = {from(beg.mom.x, 0), from(beg.mom.y, 0), from(beg.mom.z, 0)};
+
+    // Lanes 0-2: position, 3-5: momentum, 6-8: position, for the midpoint (the
+    // rest repeat lanes 0-8)
+    int const lane = threadIdx.x & 31;
+    int const group = (lane / 3) % 3;
+    int const c = lane % 3;
+    bool const is_mom = group == 1;
+    // Component i % 3 without an indexed (local) array
+    auto pick = [](Real3 const& v, int i) {
+        i = i >= 3 ? i - 3 : i;
+        return i == 0 ? v.x : (i == 1 ? v.y : v.z);
+    };
+    auto cross = [&](Real3 const& a, Real3 const& b) {
+        return pick(a, c + 1) * pick(b, c + 2) - pick(a, c + 2) * pick(b, c + 1);
+    };
+    double const start = is_mom ? pick(beg.mom, c) : pick(beg.pos, c);
+    double const product = warp_step_coefficients[lane] * (lane >= 26 ? step / 2 : step);
+    double mom_sq;
+    auto eval = [&](double y) {
+        Real3 const mom{from(y, 3), from(y, 4), from(y, 5)};
+        if (rhs.map)
+            rhs.field = rzmap_field(*rhs.map, Real3{from(y, 0), from(y, 1), from(y, 2)});
+        mom_sq = dot_product(mom, mom);
+        double const inv = fp64::div_inline(1.0, fp64::sqrt_inline(mom_sq));
+        double const scale = rhs.coeffi * inv;
+        double const direction = is_mom ? cross(mom, rhs.field) : pick(mom, c);
+        return (is_mom ? scale : inv) * direction;
+    };
+    auto add = [&](double* y, int i, double k) { *y = gbx_fma(from(product, i), k, *y); };
+    double const k1 = eval(start);
+    double const beg_mom_sq = mom_sq;
+    double y = start;
+    add(&y, 0, k1);
+    double const k2 = eval(y);
+    y = start;
+    add(&y, 1, k1);
+    add(&y, 2, k2);
+    double const k3 = eval(y);
+    y = start;
+    add(&y, 3, k1);
+    add(&y, 4, k2);
+    add(&y, 5, k3);
+    double const k4 = eval(y);
+    y = start;
+    add(&y, 6, k1);
+    add(&y, 7, k2);
+    add(&y, 8, k3);
+    add(&y, 9, k4);
+    double const k5 = eval(y);
+    y = start;
+    add(&y, 10, k1);
+    add(&y, 11, k2);
+    add(&y, 12, k3);
+    add(&y, 13, k4);
+    add(&y, 14, k5);
+    double const k6 = eval(y);
+    y = start;
+    add(&y, 15, k1);
+    add(&y, 16, k3);
+    add(&y, 17, k4);
+    add(&y, 18, k5);
+    add(&y, 19, k6);
+    double const k7 = eval(y);
+    result.end = {{from(y, 0), from(y, 1), from(y, 2)}, {from(y, 3), from(y, 4), from(y, 5)}};
+    // Error estimate, and the midpoint in lanes 6-8
+    int const first = group == 2 ? 26 : 20;
+    double z = group == 2 ? start : 0;
+    add(&z, first, k1);
+    add(&z, first + 1, k3);
+    add(&z, first + 2, k4);
+    add(&z, first + 3, k5);
+    add(&z, first + 4, k6);
+    add(&z, first + 5, k7);
+    // Two dot products at a time: even lanes' and odd lanes'
+    bool const odd = lane & 1;
+    if (chord_limit < INFINITY)
+    {
+        double const to_mid = z - start;
+        double const to_end = y - start;
+        Real3 const beg_mid{from(to_mid, 6), from(to_mid, 7), from(to_mid, 8)};
+        Real3 const beg_end{from(to_end, 6), from(to_end, 7), from(to_end, 8)};
+        double const component = cross(beg_end, beg_mid);
+        Real3 v{from(component, 0), from(component, 1), from(component, 2)};
+        if (odd)
+            v = beg_end;
+        double const square = dot_product(v, v);
+        result.dchord = gbx::sqrt(div(from(square, 0), from(square, 1)));
+        if (result.dchord > chord_limit)
+            return result;
+    }
+    int const part = odd ? 3 : 0;
+    Real3 const err{from(z, part), from(z, part + 1), from(z, part + 2)};
+    double const ratio = div(dot_product(err, err), odd ? beg_mom_sq : ipow<2>(step));
+    result.rel_err_sq = max_of(from(ratio, 0), from(ratio, 1));
+    return result;
+}
+
+//! A value that the compiler does not know (there is one warp_step for all lanes)
+__device__ __forceinline__ bool opaque(int value)
+{
+    asm volatile("" : "+r"(value));
+    return value;
+}
+
+//! Steps of lane 0's track until it is through
+__device__ __forceinline__ void help_field_warp()
+{
+    bool active = false;
+    UniformFieldEquation rhs{};
+    OdeState beg{};
+    do
+    {
+        active = warp_step(opaque(false), rhs, 0, beg, 0).active;
+    } while (active);
+}
+
+//! Lane 0, after its track: let the helpers go
+__device__ __forceinline__ void end_field_warp()
+{
+    warp_step(opaque(false), UniformFieldEquation{}, 0, OdeState{}, 0);
+}
+#endif
+
 //---------------------------------------------------------------------------//
 // Field driver
 //---------------------------------------------------------------------------//
@@ -224,6 +423,7 @@ class DormandPrinceStep
 //! One c3-like event of 20 particles 516 -> 478 ms, 7 with detector hits 84 -> 80
 //! ms, against the estimate and midpoint of every step and a copy of the step for
 //! each use.
+template<bool Warp>
 class FieldDriver
 {
   public:
@@ -288,10 +488,28 @@ class FieldDriver
         size_type tries = 0;
         for (;;)
         {
-            DormandPrinceStep<Equation> const rk(rhs, taken, result.state);
+            DormandPrinceStep<Equation> rk;
+            WarpStep warp;
+            double const chord_limit = opt_.delta_chord + FieldOptions::dchord_tol;
+            if constexpr (Warp)
+            {
+#if defined(__CUDA_ARCH__)
+                warp = warp_step(opaque(true),
+                                 rhs_,
+                                 taken,
+                                 result.state,
+                                 turn == Turn::chord ? chord_limit : INFINITY);
+#endif
+            }
+            else
+            {
+                rk.take(rhs, taken, result.state);
+                warp.end = rk.end_state();
+            }
+            OdeState const& end_state = warp.end;
             if (turn == Turn::minimum)
             {
-                result.state = rk.end_state();
+                result.state = end_state;
                 result.step = step;
                 return result;
             }
@@ -299,8 +517,9 @@ class FieldDriver
             {
                 Real3 const& beg_pos = result.state.pos;
                 double const dchord
-                    = distance_chord(beg_pos, rk.mid_pos(beg_pos), rk.end_state().pos);
-                if (dchord > opt_.delta_chord + FieldOptions::dchord_tol)
+                    = Warp ? warp.dchord
+                           : distance_chord(beg_pos, rk.mid_pos(beg_pos), end_state.pos);
+                if (dchord > chord_limit)
                 {
                     // From chord_far on the factor is the smallest one
                     double scale = FieldOptions::min_chord_shrink;
@@ -314,7 +533,10 @@ class FieldDriver
                         continue;
                 }
             }
-            double const err_sq = this->step_err_sq(rk.error(), taken, result.state.mom);
+            double const rel_err
+                = Warp ? warp.rel_err_sq : rel_err_sq(rk.error(), taken, result.state.mom);
+            // Scaled error of a step: above 1 the step is rejected
+            double const err_sq = div(rel_err, ipow<2>(opt_.epsilon_rel_max));
             if (turn == Turn::chord)
             {
                 if (taken < step)
@@ -323,7 +545,7 @@ class FieldDriver
                 }
                 if (!(err_sq > 1))
                 {
-                    result.state = rk.end_state();
+                    result.state = end_state;
                     result.step = taken;
                     return result;
                 }
@@ -356,7 +578,7 @@ class FieldDriver
                     h = min_of(max_of(taken * scale, opt_.minimum_step),
                                end_curve_length - curve_length);
                 }
-                result.state = rk.end_state();
+                result.state = end_state;
                 if (done || --remaining_steps <= 0)
                 {
                     result.step = min_of(curve_length, end_curve_length);
@@ -378,13 +600,6 @@ class FieldDriver
         errpos2 = div(errpos2, ipow<2>(step));
         errvel2 = div(errvel2, dot_product(mom, mom));
         return max_of(errpos2, errvel2);
-    }
-
-    //! Scaled error of a step: above 1 the step is rejected
-    GBX_FORCEINLINE double
-    step_err_sq(OdeState const& err_state, double step, Real3 const& mom) const
-    {
-        return div(rel_err_sq(err_state, step, mom), ipow<2>(opt_.epsilon_rel_max));
     }
 
     static GBX_FORCEINLINE double distance_chord(Real3 const& beg_pos,
@@ -419,8 +634,10 @@ inline unsigned long long safe_ball_mismatches = 0;
 //! split into its set-up, one substep of its loop and its completion so that
 //! a kernel can interleave the substeps of different tracks. Running
 //! init(), then substep() until done(), then finish() is the reference's
-//! sequence of operations. RoundX is the mixed-precision driver's.
-template<bool RoundX = true>
+//! sequence of operations. RoundX is the mixed-precision driver's. Warp: this is
+//! lane 0 of a warp whose lanes take the FP64 driver's steps together, the others
+//! in help_field_warp().
+template<bool RoundX = true, bool Warp = false>
 class FieldPropagation
 {
   public:
@@ -648,7 +865,7 @@ class FieldPropagation
   public:
 
   private:
-    std::conditional_t<sizeof(real_type) == sizeof(double), FieldDriver, MixedFieldDriver<RoundX>>
+    std::conditional_t<sizeof(real_type) == sizeof(double), FieldDriver<Warp>, MixedFieldDriver<RoundX>>
         driver_;
     OdeState state_;
     Propagation result_;
