@@ -208,13 +208,21 @@ class DormandPrinceStep
     OdeState end_;
 };
 
+//! What a warp is to take, and what the length that goes with it is
+enum class WarpTask
+{
+    none,  //!< No step: the helpers are done
+    chord,  //!< A step and its chord; its error unless that is above the length
+    error,  //!< A step and its error, its position's relative to the length
+};
+
 //! A step taken by a warp: its end, and the two numbers by which the driver
 //! accepts it
 struct WarpStep
 {
     OdeState end;
-    double dchord;  //!< Distance of the midpoint from the chord, if asked for
-    double rel_err_sq;  //!< Relative squared error, unless the chord is too far
+    double dchord;  //!< Distance of the midpoint from the chord (WarpTask::chord)
+    double rel_err_sq;  //!< Relative squared error (not of a chord too far)
     bool active;  //!< A step was taken
 };
 
@@ -256,8 +264,7 @@ static __device__ double const warp_step_coefficients[32] = {
     double(11237099.) / double(235043384.)};
 
 //! One Dormand-Prince step of one track by the 32 lanes of its warp, which all call
-//! this: lane 0 with the track's arguments, the others with 'active' alone looked
-//! at in lane 0 (no step, and the helpers are done, if it is false).
+//! this; only lane 0's arguments count.
 //!
 //! On GB300 an FP64 instruction takes its warp 64 cycles whatever its lanes do, and
 //! none overlaps another. With few tracks, each in a warp of its own, three lanes
@@ -269,16 +276,17 @@ static __device__ double const warp_step_coefficients[32] = {
 //! of 20 particles in the CMS-like detector 458 -> 363 ms, 7 with detector hits 77 -> 65
 //! ms, 300 electrons in the calorimeter 230 -> 224.5 ms.
 __device__ __noinline__ WarpStep warp_step(
-    bool active, UniformFieldEquation rhs, double step, OdeState beg, double chord_limit)
+    WarpTask task, UniformFieldEquation rhs, double step, OdeState beg, double length)
 {
     auto from = [](double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); };
     WarpStep result;
     __syncwarp();
-    result.active = __shfl_sync(0xffffffffu, int(active), 0);
+    task = static_cast<WarpTask>(__shfl_sync(0xffffffffu, int(task), 0));
+    result.active = task != WarpTask::none;
     if (!result.active)
         return result;
     step = from(step, 0);
-    chord_limit = from(chord_limit, 0);
+    length = from(length, 0);
     rhs.coeffi = from(rhs.coeffi, 0);
     rhs.field = {from(rhs.field.x, 0), from(rhs.field.y, 0), from(rhs.field.z, 0)};
     rhs.map = reinterpret_cast<RZMapData const*>(
@@ -360,7 +368,7 @@ __device__ __noinline__ WarpStep warp_step(
     add(&z, first + 5, k7);
     // Two dot products at a time: even lanes' and odd lanes'
     bool const odd = lane & 1;
-    if (chord_limit < INFINITY)
+    if (task == WarpTask::chord)
     {
         double const to_mid = z - start;
         double const to_end = y - start;
@@ -372,21 +380,23 @@ __device__ __noinline__ WarpStep warp_step(
             v = beg_end;
         double const square = dot_product(v, v);
         result.dchord = gbx::sqrt(div(from(square, 0), from(square, 1)));
-        if (result.dchord > chord_limit)
+        if (result.dchord > length)
             return result;
+        length = step;
     }
     int const part = odd ? 3 : 0;
     Real3 const err{from(z, part), from(z, part + 1), from(z, part + 2)};
-    double const ratio = div(dot_product(err, err), odd ? beg_mom_sq : ipow<2>(step));
+    double const ratio = div(dot_product(err, err), odd ? beg_mom_sq : ipow<2>(length));
     result.rel_err_sq = max_of(from(ratio, 0), from(ratio, 1));
     return result;
 }
 
 //! A value that the compiler does not know (there is one warp_step for all lanes)
-__device__ __forceinline__ bool opaque(int value)
+__device__ __forceinline__ WarpTask opaque(WarpTask task)
 {
+    int value = static_cast<int>(task);
     asm volatile("" : "+r"(value));
-    return value;
+    return static_cast<WarpTask>(value);
 }
 
 //! Steps of lane 0's track until it is through
@@ -397,14 +407,14 @@ __device__ __forceinline__ void help_field_warp()
     OdeState beg{};
     do
     {
-        active = warp_step(opaque(false), rhs, 0, beg, 0).active;
+        active = warp_step(opaque(WarpTask::none), rhs, 0, beg, 0).active;
     } while (active);
 }
 
 //! Lane 0, after its track: let the helpers go
 __device__ __forceinline__ void end_field_warp()
 {
-    warp_step(opaque(false), UniformFieldEquation{}, 0, OdeState{}, 0);
+    warp_step(opaque(WarpTask::none), UniformFieldEquation{}, 0, OdeState{}, 0);
 }
 #endif
 
@@ -494,11 +504,12 @@ class FieldDriver
             if constexpr (Warp)
             {
 #if defined(__CUDA_ARCH__)
-                warp = warp_step(opaque(true),
+                bool const chord = turn == Turn::chord;
+                warp = warp_step(opaque(chord ? WarpTask::chord : WarpTask::error),
                                  rhs_,
                                  taken,
                                  result.state,
-                                 turn == Turn::chord ? chord_limit : INFINITY);
+                                 chord ? chord_limit : taken);
 #endif
             }
             else
@@ -528,9 +539,19 @@ class FieldDriver
                         scale = max_of(gbx::sqrt(div(opt_.delta_chord, dchord)),
                                        FieldOptions::min_chord_shrink);
                     }
+                    double const tried = taken;
                     taken *= scale;
                     if (--remaining_steps > 0)
                         continue;
+                    // The last trial stands whatever its chord: by its error over
+                    // the length that would have been next
+                    if constexpr (Warp)
+                    {
+#if defined(__CUDA_ARCH__)
+                        warp = warp_step(
+                            opaque(WarpTask::error), rhs_, tried, result.state, taken);
+#endif
+                    }
                 }
             }
             double const rel_err
