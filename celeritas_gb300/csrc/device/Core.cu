@@ -1194,8 +1194,22 @@ void ActionSequence::reset_action_times()
     launches_.assign(num_ids_, 0);
 }
 
+//! Throw if the state's steps cannot sort its tracks
+static void check_sort(CoreParams const& params, CoreState const& state)
+{
+    unsigned int const order = params.host().scalars.track_order;
+    if (state.context().sort_enabled
+        && (sorts_along_step(order) || sorts_step_limit(order)
+            || order == track_order_reindex_status
+            || order == track_order_reindex_particle_type))
+    {
+        check_sort_bins(state.context());
+    }
+}
+
 void ActionSequence::step(CoreParams const& params, CoreState& state) const
 {
+    check_sort(params, state);
     if (!timing_)
     {
         // The model actions follow one another and a track interacts by one of
@@ -1280,6 +1294,8 @@ void Stepper::clear_graphs()
 void Stepper::build_graph()
 {
     int const k = state_->context().sort_enabled ? 1 : 0;
+    // (an exception in the capture would leave the stream in it)
+    check_sort(*params_, *state_);
     GBX_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     actions_->step(*params_, *state_);
     GBX_CUDA(cudaStreamEndCapture(stream_, &graph_[k]));

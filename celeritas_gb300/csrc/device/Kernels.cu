@@ -760,35 +760,32 @@ __global__ __launch_bounds__(sort_block_size) void sort_scatter_kernel(
 {
     begin_dependent();
     constexpr unsigned int num_warps = sort_block_size / 32;
-    extern __shared__ size_type warp_hist[];  // [num_warps][num_bins], [num_bins]
+    extern __shared__ size_type warp_hist[];  // [num_warps][num_bins]
     size_type const nb = srt.num_bins;
-    size_type* const bin_base = warp_hist + num_warps * nb;
-    if (threadIdx.x < 32)
+    unsigned int const lane = threadIdx.x & 31u;
+    unsigned int const warp = threadIdx.x >> 5;
+    // First position of this thread's bin (there are no more bins than threads):
+    // exclusive scan of the totals
+    size_type bin_base = 0;
+    if (warp * 32 < nb)
     {
-        // First position of each bin: exclusive scan of the totals
-        size_type before = 0;
-        for (size_type first = 0; first < nb; first += 32)
+        for (size_type b = lane; b < warp * 32; b += 32)
+            bin_base += srt.bin_totals[b];
+        bin_base = __reduce_add_sync(0xffffffffu, bin_base);
+        size_type const v = threadIdx.x < nb ? srt.bin_totals[threadIdx.x] : 0;
+        size_type incl = v;
+        for (unsigned int off = 1; off < 32; off <<= 1)
         {
-            size_type const b = first + threadIdx.x;
-            size_type const v = b < nb ? srt.bin_totals[b] : 0;
-            size_type incl = v;
-            for (unsigned int off = 1; off < 32; off <<= 1)
-            {
-                size_type const n = __shfl_up_sync(0xffffffffu, incl, off);
-                if (threadIdx.x >= off)
-                    incl += n;
-            }
-            if (b < nb)
-            {
-                bin_base[b] = before + incl - v;
-                if (blockIdx.x == 0)
-                    offsets[b] = before + incl - v;
-            }
-            before += __shfl_sync(0xffffffffu, incl, 31);
+            size_type const n = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off)
+                incl += n;
         }
-        if (blockIdx.x == 0 && threadIdx.x == 0)
-            offsets[nb] = s.size;
+        bin_base += incl - v;
+        if (blockIdx.x == 0 && threadIdx.x < nb)
+            offsets[threadIdx.x] = bin_base;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        offsets[nb] = s.size;
     for (size_type i = threadIdx.x; i < num_warps * nb; i += blockDim.x)
         warp_hist[i] = 0;
     __syncthreads();
@@ -796,26 +793,24 @@ __global__ __launch_bounds__(sort_block_size) void sort_scatter_kernel(
     bool const valid = slot < s.size;
     size_type const k = valid ? sort_key(s, srt, key, slot) : nb;
     unsigned int const peers = __match_any_sync(0xffffffffu, k);
-    unsigned int const lane = threadIdx.x & 31u;
-    unsigned int const warp = threadIdx.x >> 5;
     unsigned int const lower = peers & ((1u << lane) - 1u);
     if (valid && lower == 0)
         warp_hist[warp * nb + k] = __popc(peers);
     __syncthreads();
-    for (size_type b = threadIdx.x; b < nb; b += blockDim.x)
+    if (threadIdx.x < nb)
     {
-        size_type acc = 0;
+        size_type acc = bin_base;
         for (unsigned int w = 0; w < num_warps; ++w)
         {
-            size_type const c = warp_hist[w * nb + b];
-            warp_hist[w * nb + b] = acc;
+            size_type const c = warp_hist[w * nb + threadIdx.x];
+            warp_hist[w * nb + threadIdx.x] = acc;
             acc += c;
         }
     }
     __syncthreads();
     if (valid)
     {
-        size_type const pos = bin_base[k] + srt.block_hist[k * srt.num_blocks + blockIdx.x]
+        size_type const pos = srt.block_hist[k * srt.num_blocks + blockIdx.x]
                               + warp_hist[warp * nb + k] + __popc(lower);
         s.track_slots[pos] = slot;
     }
@@ -1469,14 +1464,23 @@ void launch_kill_active(LaunchContext const& ctx, cudaStream_t stream)
         ctx.params, ctx.state);
 }
 
+void check_sort_bins(LaunchContext const& ctx)
+{
+    if (ctx.sort.num_bins > max_sort_bins)
+        throw std::runtime_error("too many actions and materials for the track sort: "
+                                 + std::to_string(ctx.sort.num_bins) + " bins, at most "
+                                 + std::to_string(max_sort_bins));
+}
+
 void launch_sort_tracks(LaunchContext const& ctx, SortKey key, cudaStream_t stream)
 {
+    check_sort_bins(ctx);
     SortScratch const& srt = ctx.sort;
     launch(sort_count_kernel, srt.num_blocks, sort_block_size,
            srt.num_bins * sizeof(size_type), stream, ctx.state, srt, key);
     launch(sort_scan_kernel, srt.num_bins, 1024, 0, stream, srt);
     launch(sort_scatter_kernel, srt.num_blocks, sort_block_size,
-           (sort_block_size / 32 + 1) * srt.num_bins * sizeof(size_type), stream,
+           (sort_block_size / 32) * srt.num_bins * sizeof(size_type), stream,
            ctx.state, srt, key, sort_offsets(ctx, key));
 }
 

@@ -41,7 +41,7 @@ struct SortScratch
 {
     size_type* block_hist;  //!< [num_bins * num_blocks]
     size_type* bin_totals;  //!< [num_bins]
-    //! num_actions + num_materials + 1 (last: invalid action)
+    //! num_actions + 2 * num_materials + 1 (last: invalid action)
     size_type num_bins;
     size_type num_blocks;
     size_type num_actions;
@@ -182,6 +182,12 @@ int persistent_along_blocks(int threads_per_block);
 void launch_count_event_live(LaunchContext const& ctx,
                              size_type num_events,
                              cudaStream_t stream);
+//! Largest number of sort bins: the scatter's counts of every warp and bin take the
+//! 48 KB of shared memory that a block has without opting in to more
+constexpr size_type max_sort_bins
+    = 48 * 1024 / ((sort_block_size / 32) * sizeof(size_type));
+//! Throw if the state's bins are more than the sort can take
+void check_sort_bins(LaunchContext const& ctx);
 //! Stable counting sort of the track slots by action (SortTracksAction):
 //! fills state.track_slots and state.action_offsets
 void launch_sort_tracks(LaunchContext const& ctx, SortKey key, cudaStream_t stream);
