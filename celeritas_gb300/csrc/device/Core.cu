@@ -1296,9 +1296,12 @@ void Stepper::build_graph()
     int const k = state_->context().sort_enabled ? 1 : 0;
     // (an exception in the capture would leave the stream in it)
     check_sort(*params_, *state_);
+    // Primaries in wait are for the next step alone, not for each replay
+    size_type const pending = state_->hold_pending_primaries();
     GBX_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     actions_->step(*params_, *state_);
     GBX_CUDA(cudaStreamEndCapture(stream_, &graph_[k]));
+    state_->restore_pending_primaries(pending);
     GBX_CUDA(cudaGraphInstantiate(&graph_exec_[k], graph_[k], 0));
 }
 

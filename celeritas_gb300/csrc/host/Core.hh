@@ -16,6 +16,7 @@
 #include <string>
 #include <string_view>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "../device/Kernels.cuh"
@@ -169,6 +170,9 @@ class CoreState
     void generate_primaries(PrimaryGeneratorData gen);
     size_type pending_primaries() const { return pending_primaries_; }
     void clear_pending_primaries() { pending_primaries_ = 0; }
+    //! Set the primaries in wait aside, and bring them back
+    size_type hold_pending_primaries() { return std::exchange(pending_primaries_, 0); }
+    void restore_pending_primaries(size_type n) { pending_primaries_ = n; }
 
     //! Copy the device counters to the host (synchronizes the stream)
     Counters counters() const;
