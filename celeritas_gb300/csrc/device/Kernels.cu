@@ -955,7 +955,7 @@ __global__ __launch_bounds__(block_size, 1) void along_charged_warp_kernel(
     end_field_warp();
 }
 
-//! Before a charged along-step in a field: no track claimed, none listed
+//! Before the list below or the persistent kernel: no track claimed, none listed
 __global__ void clear_along_work_kernel(AlongWork work)
 {
     begin_dependent();
@@ -1262,8 +1262,10 @@ void launch_along_step(LaunchContext const& ctx,
         size_type warp_tracks = 0;
         if (p.has_field)
         {
-            launch(clear_along_work_kernel, 1, 1, 0, stream, ctx.along_work);
-            if (!range.offsets || reindexes_all(p.track_order))
+            bool const list = !range.offsets || reindexes_all(p.track_order);
+            if (list || ctx.persistent_blocks > 0)
+                launch(clear_along_work_kernel, 1, 1, 0, stream, ctx.along_work);
+            if (list)
             {
                 launch(list_charged_kernel, nb, block_size, 0, stream, p, ctx.state,
                        ctx.along_work);

@@ -32,3 +32,26 @@ def test_counting_leaves_pending_primaries(gb):
     steps = transport(False)
     assert steps[0][0] == 2 and steps[-1][3] == 0
     assert transport(True) == steps
+
+
+# More than without a field: the FP64 build's kernel for few tracks, the list of the
+# charged tracks where none is sorted, and the clearing of what the list and the
+# persistent kernel count with
+@pytest.mark.parametrize("precision, order, persistent, more", [
+    ("double", "reindex_both_action", 0, 1),
+    ("double", "reindex_both_action", 1, 1),
+    ("double", "none", 0, 3),
+    ("mixed", "reindex_both_action", 0, 0),
+    ("mixed", "reindex_both_action", 1, 1),
+    ("mixed", "none", 0, 2),
+    ("mixed", "reindex_particle_type", 1, 2),
+])
+def test_launches_for_a_field(gb, precision, order, persistent, more):
+    def kernels(field):
+        params = gb.Params(gb.physics_file("calo"), "calo", field_tesla=(0.0, 0.0, field),
+                           msc=True, track_order=order, precision=precision)
+        st = gb.Stepper(params, 4096, seed=1)
+        st.set_tuning(along_persistent=persistent)
+        return st.step_kernels()
+
+    assert kernels(1.0) - kernels(0.0) == more
