@@ -18,6 +18,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 
 #include "../gbx/TrackInit.hh"
 
@@ -935,6 +936,8 @@ along_step_sorted_kernel(ParamsData p,
 //! the FP64 units are shared (300 electrons in the calorimeter with at most 1, 2, 4, 8
 //! tracks per SM: 239, 237, 234, 233 ms). A kernel of its own: in one with
 //! along_step_sorted_kernel it makes that one 4% slower (233 against 224.5 ms).
+//! Real: the build's real_type, for the launch that only the FP64 build has.
+template<class Real>
 __global__ __launch_bounds__(block_size, 1) void along_charged_warp_kernel(
     ParamsData p, StateData s, SlotRange range, size_type warp_tracks)
 {
@@ -1234,6 +1237,25 @@ void launch_pre_step(LaunchContext const& ctx, cudaStream_t stream)
 }
 
 
+//! Charged along-step of few tracks by a warp each; returns up to how many (none in
+//! the mixed build). One track per warp of a block on every SM; the persistent
+//! kernel takes all its tracks itself.
+template<class Real>
+size_type launch_along_warps(LaunchContext const& ctx, SlotRange const& range, cudaStream_t stream)
+{
+    if constexpr (std::is_same_v<Real, double>)
+    {
+        if (ctx.persistent_blocks == 0)
+        {
+            size_type const warp_tracks = ctx.num_sms * (block_size / 32);
+            launch(along_charged_warp_kernel<Real>, ctx.num_sms, block_size, 0, stream,
+                   ctx.params, ctx.state, range, warp_tracks);
+            return warp_tracks;
+        }
+    }
+    return 0;
+}
+
 void launch_along_step(LaunchContext const& ctx,
                        size_type action,
                        cudaStream_t stream)
@@ -1273,14 +1295,7 @@ void launch_along_step(LaunchContext const& ctx,
             }
             spread_blocks = ctx.num_sms * max_of(1u, spread_threads / abs);
             blocks = max_of<unsigned int>(blocks, spread_blocks);
-            // One track per warp of a block on every SM; the persistent kernel
-            // takes all its tracks itself
-            if (sizeof(real_type) == sizeof(double) && ctx.persistent_blocks == 0)
-            {
-                warp_tracks = ctx.num_sms * (block_size / 32);
-                launch(along_charged_warp_kernel, ctx.num_sms, block_size, 0, stream, p,
-                       ctx.state, range, warp_tracks);
-            }
+            warp_tracks = launch_along_warps<real_type>(ctx, range, stream);
         }
         if (p.has_field && ctx.persistent_blocks > 0)
         {

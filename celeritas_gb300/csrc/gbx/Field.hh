@@ -661,6 +661,9 @@ inline unsigned long long safe_ball_mismatches = 0;
 template<bool RoundX = true, bool Warp = false>
 class FieldPropagation
 {
+    static_assert(!Warp || sizeof(real_type) == sizeof(double),
+                  "only the FP64 driver takes steps with its warp's lanes");
+
   public:
     GBX_FORCEINLINE FieldPropagation(FieldOptions const& opt,
                                      UniformFieldEquation const& rhs)
