@@ -548,8 +548,7 @@ class FieldDriver
                     if constexpr (Warp)
                     {
 #if defined(__CUDA_ARCH__)
-                        warp = warp_step(
-                            opaque(WarpTask::error), rhs_, tried, result.state, taken);
+                        warp = last_warp_step(rhs_, tried, result.state, taken);
 #endif
                     }
                 }
@@ -611,6 +610,16 @@ class FieldDriver
             tries = opt_.max_nsteps;
         }
     }
+
+#if defined(__CUDACC__)
+    //! A used-up search's last trial with its error over another length (out of line:
+    //! beside the loop's own step it takes an event of 20 particles 0.3% longer)
+    static __device__ __noinline__ WarpStep
+    last_warp_step(UniformFieldEquation rhs, double step, OdeState beg, double length)
+    {
+        return warp_step(opaque(WarpTask::error), rhs, step, beg, length);
+    }
+#endif
 
     static GBX_FORCEINLINE double rel_err_sq(OdeState const& err_state,
                                              double step,
