@@ -7,11 +7,15 @@
 // 1.4, an integer add 1.5 and 0.35. Each function here reduces its argument exactly
 // in 64- and 128-bit integers, sums a Taylor series whose terms are held to as
 // many bits as they contribute (32 or 64), and rounds the 128-bit result when an
-// error of 2^-66 relative (2^-64 for sin and cos, 2^-62 for expm1; the terms
-// dropped and truncated sum to less than a quarter of it) cannot change the
-// rounding. Otherwise, for about one argument in 2^13 (log, log1p, exp), 2^11 (sin,
-// cos) or 2^9 (expm1), and outside the range covered, it returns false and the
-// caller evaluates in double-doubles.
+// error of 2^-66 (exp, log, log1p), 2^-64 (sin, cos) or 2^-62 (expm1) of the power of two
+// at or below the result cannot change the rounding. Otherwise, for about one argument
+// in 2^13, 2^11 or 2^9, and outside the range covered, it returns false and the caller
+// evaluates in double-doubles.
+//
+// The truncations of every operation, the rounded coefficients and the terms dropped,
+// all at their worst and in one direction, sum to at most these parts of the error
+// allowed: 0.48 (exp), 0.65 (log, log1p; near |log| = 2^-7), 0.62 (sin, cos; near pi/4) and
+// 0.59 (expm1; below 2^-12).
 //
 // Sizes: 128-entry tables as Libm.hh's (log: C_j 2^-10 near 1/m, so that m C_j - 1
 // is exact in 64 bits; exp: 2^(j/128)) leave |z| <= 2^-7 and |r| <= 2^-8.5, of which
@@ -106,11 +110,25 @@ GBX_FORCEINLINE u128 mul_u32(u32 k, Words w)
     return make128(p2, (p1 << 32) | static_cast<u32>(p0));
 }
 
+#if defined(GBX_LIBM_RECORD)
+//! What round_result() was last given (host tests)
+struct Rounded
+{
+    u128 v;
+    int e;
+    int bits;
+};
+inline Rounded last_rounded{};
+#endif
+
 //! v 2^-127 times 2^e, v in [2^127, 2^128), with its sign, rounded to a double;
-//! false when an error of 2^-Bits v could change the rounding
+//! false when an error of 2^-Bits times 2^127 in v could change the rounding
 template<int Bits>
 GBX_FORCEINLINE bool round_result(u128 v, int e, u64 sign, u64* y)
 {
+#if defined(GBX_LIBM_RECORD)
+    last_rounded = {v, e, Bits};
+#endif
     u64 const hi = static_cast<u64>(v >> 64);
     // The 32 bits below the 53-bit significand (half: 2^31), the error in them
     u32 const rest = static_cast<u32>((hi & 0x7ffu) << 21)
@@ -133,9 +151,15 @@ GBX_FORCEINLINE i64 log1p_series(i64 z)
     t = c8 - (fp64::mul_hi_s(zs, t) >> 6);
     t = c7 - (fp64::mul_hi_s(zs, t) >> 6);
     t = c6 - (fp64::mul_hi_s(zs, t) >> 5);  // times 2^33
-    // From here times 2^63
+    // From here times 2^63. zs is up to 2^-38 below z, which raises w by up to 2^25 / 6;
+    // the last product of the series lowers it by up to 2^-69, which is 2^22 in w at
+    // |z| = 2^-7. Half of each is taken off here, so that the errors near there, the
+    // largest, are on both sides: 0.65 of the error allowed instead of 0.90 (and a
+    // wider one costs 100 electrons of 1 GeV in the calorimeter 2%: more arguments are left
+    // to the double-doubles).
     constexpr i64 one = 0x7fffffffffffffffll;
-    i64 w = one / 5 - ((static_cast<i64>(zs) * t) >> 8);
+    constexpr i64 center = (1ll << 24) / 6 + (1ll << 21);
+    i64 w = one / 5 - center - ((static_cast<i64>(zs) * t) >> 8);
     w = one / 4 - (mulhi(z, w) >> 6);
     w = one / 3 - (mulhi(z, w) >> 6);
     w = one / 2 - (mulhi(z, w) >> 6);
