@@ -410,7 +410,11 @@ struct FieldOptions
         chord_far = static_cast<float>(delta_chord * 4.01);
         if (!(chord_far > chord_limit))
             chord_far = chord_limit;
-        double const inv = 1 / (epsilon_rel_max * epsilon_rel_max);
+        double inv = 1 / (epsilon_rel_max * epsilon_rel_max);
+        // Below this the second float loses bits to FP32's underflow: a NaN leaves
+        // every norm to FP64 (as an overflow does)
+        if (inv < 0x1p-100)
+            inv = NAN;
         inv_tolerance[0] = static_cast<float>(inv);
         inv_tolerance[1] = static_cast<float>(inv - double(inv_tolerance[0]));
     }
