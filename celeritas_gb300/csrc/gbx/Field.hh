@@ -895,9 +895,6 @@ class FieldPropagation
         return dsq < room * room;
     }
 
-  public:
-
-  private:
     std::conditional_t<sizeof(real_type) == sizeof(double), FieldDriver<Warp>, MixedFieldDriver<RoundX>>
         driver_;
     OdeState state_;
@@ -910,22 +907,5 @@ class FieldPropagation
     double remaining_;
     short remaining_substeps_;
 };
-
-//! Propagate a charged track up to 'step' along its curved trajectory,
-//! stopping at the first boundary crossing (FieldPropagator::operator())
-GBX_FUNCTION Propagation propagate_in_field(FieldOptions const& opt,
-                                            UniformFieldEquation const& rhs,
-                                            double momentum,
-                                            GeoTrackView& geo,
-                                            double step)
-{
-    FieldPropagation<> fp(opt, rhs);
-    fp.init(geo, momentum, step);
-    do
-    {
-        fp.substep(geo);
-    } while (!fp.done());
-    return fp.finish(geo);
-}
 
 }  // namespace gbx
