@@ -790,6 +790,9 @@ def run_gb300(args, wl):
         "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                      "peak_source": peak_kind, "launch_ms": act["ms_per_launch"],
+                     "timed": "each action by itself, eagerly (the steps of 'value' replay "
+                              "a graph with one launch for all models, one for boundary and "
+                              "cut)",
                      "algorithmic_bytes_per_launch": act["bytes_per_launch"],
                      "actions": {k: {"ms": round(v["ms_per_launch"], 4),
                                      "GB/s": round(v["bytes_per_launch"]

@@ -1263,7 +1263,9 @@ void launch_along_step(LaunchContext const& ctx,
     // Each along-step action runs a kernel compiled for that action only,
     // over its sorted range or (sorting off) over all slots; the grid covers
     // the largest range. Sorted and unsorted orders thus run the same code,
-    // and a track's result does not depend on the track order.
+    // and a track's result does not depend on the track order. (In the mixed build
+    // it may on the kernel: the persistent one rounds one square of steps of at most the
+    // minimum length differently, MixedFieldDriver's RoundX.)
     ParamsData const& p = ctx.params;
     unsigned int const nb = num_blocks_for(ctx.state.size);
     unsigned int const abs = static_cast<unsigned int>(ctx.along_block_size);

@@ -16,12 +16,12 @@
 //   them, and from FP64 in the few cases left, so that both are what FP64 gives.
 // - A chord far too long halves the step without the division and square root
 //   that would give a factor below one half.
-// - 1 / sqrt(|p|^2) of the stages takes 60 cycles instead of 137 (inv_sqrt).
+// - 1 / sqrt(|p|^2) of the stages takes 55 cycles instead of 109 (inv_sqrt).
 // - FP32 arithmetic is spelled out (fma or not), so that no change around it
 //   changes its contraction; where the compiler had contracted the copies of the
 //   step in two ways both are kept (round_x).
-// A Runge-Kutta step takes 1250 cycles of one track's time, of which the seven
-// stages' dependent chain is about 900. A 13-event c3 batch went from 500 to 386
+// A step's stages, error estimate and chord take one track 780 cycles, most of them the
+// seven stages' dependent chain. A 13-event c3 batch went from 500 to 386
 // ms with this, four events in the field map from 555 to 403 ms, every track's
 // state the same after every step.
 #pragma once
@@ -105,12 +105,14 @@ struct Pair
     float lo;
 };
 
+//! Exact sum (Knuth's)
 GBX_FORCEINLINE Pair two_sum(float a, float b)
 {
     float const s = add(a, b);
     float const t = sub(s, a);
     return {s, add(sub(a, sub(s, t)), sub(b, t))};
 }
+//! Exact sum for |a| >= |b| (Dekker's)
 GBX_FORCEINLINE Pair fast_two_sum(float a, float b)
 {
     float const s = add(a, b);
@@ -426,8 +428,10 @@ GBX_FORCEINLINE double new_step_scale(bool above,
 //! and again. The FP64 addition of an accepted step to the position is left
 //! to the next turn, beside that step's FP32 work.
 //!
-//! RoundX: which square steps of at most the minimum length round by itself
-//! (each along-step kernel keeps its own).
+//! RoundX: which square steps of at most the minimum length round by itself. The
+//! one-thread-per-track kernel (true) and the persistent one (false) differ in it, as the
+//! compiler had contracted them, so that either keeps its results; a track with such
+//! a step may differ in the last bits between the two.
 template<bool RoundX>
 class MixedFieldDriver
 {

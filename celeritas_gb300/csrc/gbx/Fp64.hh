@@ -17,8 +17,8 @@
 // remainder. A quotient or a root of 53-bit numbers is never a midpoint of two
 // 53-bit numbers, so the first 54 bits decide the rounding.
 //
-// Both are functions of their own: 307 and 333 cycles of a warp with the call
-// (28 and 30 of the SM), against 249 and 284 inlined. Inlined at their ~200 call
+// Both are functions of their own: 307 and 339 cycles of a warp with the call
+// (28 and 31 of the SM), against 250 and 283 inlined. Inlined at their ~200 call
 // sites they made a transport slower, not faster (one 100 MeV shower in FP64 14.3
 // ms against 13.3 with the hardware's operations and 12.2 with calls): with few
 // tracks a launch runs through its code once, and its time is that of fetching
